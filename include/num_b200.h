@@ -61,7 +61,10 @@ typedef struct {
  * sums from a copy of the matrix sorted by row length and stored as
  * column-major 32-row slices, lane per row (built when first selected; a
  * matrix it would pad to more than twice its nonzeros runs GATHER instead).
- * AUTO: GATHER when at least 3/4 of the nonzeros lie in row blocks without x
+ * AUTO: a matrix whose nonzeros lie on at most 16 diagonals (rows ascending,
+ * none longer than short_max) runs from its diagonal form -- masks and values
+ * by diagonal, no column indices -- with the sums of BLOCKS bit for bit, and is
+ * reported as BLOCKS; else GATHER when at least 3/4 of the nonzeros lie in row blocks without x
  * windows and no row has more than 4096 nonzeros, else BLOCKS.  The
  * autotuner times all three.  CG and the batched engine always use the
  * row-block pipeline. */

@@ -70,6 +70,22 @@ int prepare_kernel(const void* fn, int threads, size_t smem, int* ctas_per_sm) {
     return NM_OK;
 }
 
+int kernel_occupancy(const void* fn, int threads, int* ctas_per_sm) {
+    int dev = 0;
+    NM_CUDA_TRY(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> g(g_kern_mu);
+    auto key = std::make_pair(fn, dev);
+    auto it = g_kern_occ.find(key);
+    if (it == g_kern_occ.end()) {
+        int occ = 0;
+        NM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, threads, 0));
+        if (occ < 1) return fail(NM_ERR_CUDA, "kernel does not fit on an SM");
+        it = g_kern_occ.emplace(key, occ).first;
+    }
+    *ctas_per_sm = it->second;
+    return NM_OK;
+}
+
 namespace {
 std::mutex g_err_mu;
 std::unordered_map<int, std::pair<unsigned int*, unsigned int*>> g_err;  // dev -> (host, device)

@@ -7,6 +7,8 @@
 #include <stdarg.h>
 #include <stdio.h>
 
+#include <type_traits>
+
 #include "../../include/num_b200.h"
 
 namespace nm {
@@ -33,6 +35,10 @@ unsigned int* device_error_word();
 // maximum shared-memory carveout on the current device (once per device) and
 // returns how many CTAs of `threads` threads fit on one SM.
 int prepare_kernel(const void* fn, int threads, size_t smem, int* ctas_per_sm);
+
+// CTAs of `threads` threads per SM of kernel `fn` without dynamic shared
+// memory (once per device; its attributes are left alone).
+int kernel_occupancy(const void* fn, int threads, int* ctas_per_sm);
 
 // Device error codes.
 constexpr unsigned int kErrWaitTimeout = 1u;  // a bounded mbarrier wait gave up
@@ -105,6 +111,15 @@ __device__ __forceinline__ A widen(V v) { return static_cast<A>(v); }
 template <>
 __device__ __forceinline__ float widen<__nv_bfloat16, float>(__nv_bfloat16 v) {
     return __bfloat162float(v);
+}
+
+// One matrix value, read once (evict-first).
+template <typename V>
+__device__ __forceinline__ V ld_value_cs(const V* p) {
+    if constexpr (std::is_same_v<V, __nv_bfloat16>)
+        return __ushort_as_bfloat16(__ldcs(reinterpret_cast<const unsigned short*>(p)));
+    else
+        return __ldcs(p);
 }
 
 // Unfused multiply and add, so serial sums reproduce the CPU order bit for bit

@@ -147,11 +147,21 @@ int validate_csr(const int32_t* rp, const int32_t* ci, int32_t nrows, int32_t nc
     return NM_OK;
 }
 
+// The row offsets (rp_len of them) and, behind them, room for the search for a
+// diagonal form and for its masks: one allocation.
+int alloc_row_ptr(nm_csr* A, size_t rp_len) {
+    const size_t rb = (sizeof(int32_t) * rp_len + 255) & ~size_t(255);
+    NM_CUDA_TRY(cudaMalloc(&A->d_row_ptr, rb + kDiaTableBytes + 2 * size_t(A->nrows) + 256));
+    A->d_dia_room = reinterpret_cast<unsigned char*>(A->d_row_ptr) + rb;
+    return NM_OK;
+}
+
 int upload(nm_csr* A, const int32_t* rp, const int32_t* ci, const void* vals) {
     const size_t es = dtype_size(A->dtype);
     const int64_t nnz_pad = ((static_cast<int64_t>(A->nnz) + 7) & ~int64_t(7)) + 8;
     const size_t rp_len = size_t(A->nrows) + 1 + 8;
-    NM_CUDA_TRY(cudaMalloc(&A->d_row_ptr, sizeof(int32_t) * rp_len));
+    const int st = alloc_row_ptr(A, rp_len);
+    if (st != NM_OK) return st;
     NM_CUDA_TRY(cudaMalloc(&A->d_col_idx, sizeof(int32_t) * size_t(nnz_pad)));
     NM_CUDA_TRY(cudaMalloc(&A->d_values, es * size_t(nnz_pad)));
     {
@@ -218,6 +228,7 @@ int rebuild_blocks(nm_csr* A) {
             if (desc[b].xs.x < 0) gathered += desc[b].rz.w - desc[b].rz.z;
         int32_t max_row = 0;
         for (int32_t r = 0; r < A->nrows; ++r) max_row = std::max(max_row, rp[r + 1] - rp[r]);
+        A->max_row = max_row;
         const bool scattered = A->nnz > 0 && 4 * gathered >= 3 * int64_t(A->nnz) &&
                                max_row <= kWarpGatherMaxRow;
         A->warp_gather = A->tune.kernel == NM_KERNEL_GATHER ||
@@ -228,20 +239,19 @@ int rebuild_blocks(nm_csr* A) {
         const int st = build_sell(A);
         if (st != NM_OK) return st;
     }
-    if (A->d_blk) {
-        cudaFree(A->d_blk);
-        A->d_blk = nullptr;
-    }
+    // descriptors, then block boundaries, in one allocation and one copy
     if (A->d_desc) {
         cudaFree(A->d_desc);
         A->d_desc = nullptr;
+        A->d_blk = nullptr;
     }
-    NM_CUDA_TRY(cudaMalloc(&A->d_blk, sizeof(int32_t) * blk.size()));
-    NM_CUDA_TRY(cudaMalloc(&A->d_desc, sizeof(BlockDesc) * desc.size()));
-    NM_CUDA_TRY(cudaMemcpy(A->d_blk, blk.data(), sizeof(int32_t) * blk.size(),
-                           cudaMemcpyHostToDevice));
-    NM_CUDA_TRY(cudaMemcpy(A->d_desc, desc.data(), sizeof(BlockDesc) * desc.size(),
-                           cudaMemcpyHostToDevice));
+    const size_t db = sizeof(BlockDesc) * desc.size(), bb = sizeof(int32_t) * blk.size();
+    std::vector<unsigned char> both(db + bb);
+    if (db) std::memcpy(both.data(), desc.data(), db);
+    std::memcpy(both.data() + db, blk.data(), bb);
+    NM_CUDA_TRY(cudaMalloc(&A->d_desc, db + bb));
+    A->d_blk = reinterpret_cast<int32_t*>(reinterpret_cast<unsigned char*>(A->d_desc) + db);
+    NM_CUDA_TRY(cudaMemcpy(A->d_desc, both.data(), db + bb, cudaMemcpyHostToDevice));
     return NM_OK;
 }
 
@@ -254,6 +264,7 @@ int finish_create(nm_csr* A, const int32_t* rp, const int32_t* ci, const void* v
         A->h_row_ptr.assign(rp, rp + A->nrows + 1);
         A->h_col_idx.assign(ci, ci + A->nnz);
         st = rebuild_blocks(A);
+        if (st == NM_OK) st = find_dia_form(A);
     }
     if (st != NM_OK) {
         delete A;
@@ -285,13 +296,13 @@ nm_csr::~nm_csr() {
     if (d_row_ptr) cudaFree(d_row_ptr);
     if (d_col_idx) cudaFree(d_col_idx);
     if (d_values) cudaFree(d_values);
-    if (d_blk) cudaFree(d_blk);
-    if (d_desc) cudaFree(d_desc);
+    if (d_desc) cudaFree(d_desc);  // and d_blk behind it
     if (d_sell_ptr) cudaFree(d_sell_ptr);
     if (d_sell_row) cudaFree(d_sell_row);
     if (d_sell_len) cudaFree(d_sell_len);
     if (d_sell_col) cudaFree(d_sell_col);
     if (d_sell_val) cudaFree(d_sell_val);
+    if (dia.d_val) cudaFree(dia.d_val);
 }
 
 using nm::fail;
@@ -407,13 +418,14 @@ extern "C" int nm_csr_laplacian(int32_t dim, int32_t L, int dtype, nm_csr** out)
         // Same allocation and padding as an uploaded matrix.
         const int64_t nnz_pad = ((nnz + 7) & ~int64_t(7)) + 8;
         const int64_t rp_len = n + 1 + 8;
-        NM_CUDA_TRY(cudaMalloc(&A->d_row_ptr, sizeof(int32_t) * size_t(rp_len)));
+        int st = nm::alloc_row_ptr(A, size_t(rp_len));
+        if (st != NM_OK) return st;
         NM_CUDA_TRY(cudaMalloc(&A->d_col_idx, sizeof(int32_t) * size_t(nnz_pad)));
         NM_CUDA_TRY(cudaMalloc(&A->d_values, es * size_t(nnz_pad)));
         NM_CUDA_TRY(cudaMemset(A->d_col_idx + nnz, 0, sizeof(int32_t) * size_t(nnz_pad - nnz)));
         NM_CUDA_TRY(cudaMemset(static_cast<char*>(A->d_values) + es * size_t(nnz), 0,
                                es * size_t(nnz_pad - nnz)));
-        int st = nm::launch_laplacian(dim, L, dtype, A->d_row_ptr, rp_len, A->d_col_idx,
+        st = nm::launch_laplacian(dim, L, dtype, A->d_row_ptr, rp_len, A->d_col_idx,
                                       A->d_values, nullptr);
         if (st != NM_OK) return st;
         // The row-block partition is built on the host from row_ptr and the
@@ -424,7 +436,8 @@ extern "C" int nm_csr_laplacian(int32_t dim, int32_t L, int dtype, nm_csr** out)
                                cudaMemcpyDeviceToHost));
         NM_CUDA_TRY(cudaMemcpy(A->h_col_idx.data(), A->d_col_idx, sizeof(int32_t) * size_t(nnz),
                                cudaMemcpyDeviceToHost));
-        return nm::rebuild_blocks(A);
+        st = nm::rebuild_blocks(A);
+        return st == NM_OK ? nm::find_dia_form(A) : st;
     };
     const int st = build();
     if (st != NM_OK) {
@@ -492,7 +505,7 @@ extern "C" int nm_csr_set_tuning(nm_csr* A, const nm_tuning* t) {
 extern "C" int nm_csr_spmv_kernel(const nm_csr* A, int32_t* kernel) {
     nm::clear_error();
     if (!A || !kernel) return fail(NM_ERR_INVALID, "nm_csr_spmv_kernel: NULL argument");
-    *kernel = !A->warp_gather ? NM_KERNEL_BLOCKS
+    *kernel = !A->warp_gather || A->use_dia() ? NM_KERNEL_BLOCKS
               : (A->tune.kernel == NM_KERNEL_SLICED && A->sell_ready ? NM_KERNEL_SLICED
                                                                       : NM_KERNEL_GATHER);
     return NM_OK;

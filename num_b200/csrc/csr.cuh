@@ -1,11 +1,12 @@
 // csr.cuh -- internal layout of a device CSR matrix.
 //
 // HBM layout (one cudaMalloc each, 256-byte aligned):
-//   row_ptr  int32[nrows + 1 + 8]  pad = nnz
+//   row_ptr  int32[nrows + 1 + 8]  pad = nnz; behind it the room of DiaForm
 //   col_idx  int32[nnz_pad]        nnz_pad = round_up(nnz, 8) + 8, pad = column 0
 //   values   V[nnz_pad]            pad = 0
-//   blk      int32[nblk + 1]       row-block boundaries (see build_row_blocks)
 //   desc     BlockDesc[nblk]       per block rows, nonzeros and x windows
+//   blk      int32[nblk + 1]       row-block boundaries (see build_row_blocks),
+//                                  behind desc
 // The padding lets the TMA bulk copies of a block start and end on 16-byte
 // boundaries (nonzeros rounded to multiples of 8, row_ptr to multiples of 4),
 // and lets a thread load 4 consecutive nonzeros with one 16-byte access,
@@ -61,6 +62,22 @@ struct CsrView {
     int32_t coherent_x = 0;
 };
 
+// The matrix in diagonal form (dia.cuh), when it has one (ndiag > 0).
+constexpr int kDiaMax = 16;
+struct DiaForm {
+    int32_t ndiag = 0;
+    bool constant = false;  // every diagonal holds one number: cval, no d_val
+    int64_t ld = 0;
+    int32_t off[kDiaMax] = {};   // col - row, ascending
+    double cval[kDiaMax] = {};
+    void* d_mask = nullptr;  // uint8_t[nrows] up to 8 diagonals, else uint16_t[nrows]
+    void* d_val = nullptr;   // values [ndiag][ld], the matrix's type
+};
+
+// Room behind the row offsets for the search for that form (dia.cu); the masks
+// follow it there.
+constexpr size_t kDiaTableBytes = 512;
+
 // Default row-block parameters.
 constexpr int kDefaultTile = 2048;
 constexpr int kDefaultMaxRows = kThreads;
@@ -106,9 +123,10 @@ struct nm_csr {
     int32_t* d_row_ptr = nullptr;
     int32_t* d_col_idx = nullptr;
     void* d_values = nullptr;
-    int32_t* d_blk = nullptr;
+    int32_t* d_blk = nullptr;  // in d_desc's allocation
     nm::BlockDesc* d_desc = nullptr;
     int32_t nblk = 0;
+    int32_t max_row = 0;  // nonzeros of the longest row
     nm_tuning tune{};
     // Plain SpMV by the warp-gather kernel (spmv.cu): set by rebuild_blocks
     // from tune.kernel (AUTO: most nonzeros in blocks without x windows and no
@@ -129,6 +147,16 @@ struct nm_csr {
     int32_t* d_sell_len = nullptr;
     int32_t* d_sell_col = nullptr;
     void* d_sell_val = nullptr;
+    // The matrix in diagonal form, when its nonzeros lie on few diagonals
+    // (found once, when the arrays are in place); d_dia_room lies behind the
+    // row offsets in their allocation.
+    nm::DiaForm dia;
+    unsigned char* d_dia_room = nullptr;
+    // The plain SpMV runs on the diagonal form: it sums every row by one
+    // thread, as the row-block kernel does for rows up to short_max.
+    bool use_dia() const {
+        return dia.ndiag > 0 && tune.kernel == NM_KERNEL_AUTO && max_row <= tune.short_max;
+    }
     std::vector<int32_t> h_row_ptr;  // kept to rebuild the partition on retuning
     std::vector<int32_t> h_col_idx;  // kept to rebuild the x windows on retuning
     // Many-matrix handles: per-matrix row / column offsets (count + 1 each).
@@ -170,6 +198,11 @@ constexpr int32_t kSellWindow = 65536;
 // Builds A's sliced copy for the gather kernel once (spmv.cu); NM_OK also
 // when the layout would pad too much (A->sell_ready stays false).
 int build_sell(nm_csr* A);
+// Looks for A's diagonal form (dia.cu) once its arrays are on the device;
+// NM_OK also when it has none.
+int find_dia_form(nm_csr* A);
+// y = A x on the diagonal form.
+int launch_spmv_dia(const nm_csr* A, const void* x, void* y, cudaStream_t stream);
 // Drops A's cached CG workspace (its graphs hold the current descriptors).
 void reset_cg(nm_csr* A);
 // Nonzeros of the Laplacian on an L^dim grid (dim 2: 5-point, dim 3: 7-point).

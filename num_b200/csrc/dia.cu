@@ -1,0 +1,378 @@
+// dia.cu -- finding a matrix's diagonal form (dia.cuh), and its SpMV.
+#include <algorithm>
+#include <cstring>
+
+#include "dia.cuh"
+
+namespace nm {
+
+namespace {
+
+// What the search kernel finds, in device memory behind the row offsets.
+constexpr int kDiaSlots = kDiaMax + 1;         // one more than allowed: overflow
+constexpr int32_t kDiaNoOff = INT32_MIN;       // col - row is never this
+constexpr uint64_t kDiaNoVal = 0x7FF0D1A0D1A0D1A0ull;  // a signalling NaN
+struct DiaTable {
+    int32_t off[kDiaSlots];
+    uint32_t overflow;  // more than kDiaMax diagonals
+    uint32_t disorder;  // a row's columns do not ascend
+    uint32_t varying;   // some diagonal holds different numbers
+    unsigned long long pairs;  // (warp of 32 rows, diagonal) pairs with an entry
+    uint64_t val[kDiaSlots];
+};
+static_assert(sizeof(DiaTable) <= kDiaTableBytes, "table room");
+
+template <typename V>
+__device__ __forceinline__ uint64_t value_bits(V v) {
+    if constexpr (std::is_same_v<V, double>)
+        return static_cast<uint64_t>(__double_as_longlong(v));
+    else if constexpr (std::is_same_v<V, float>)
+        return __float_as_uint(v);
+    else
+        return __bfloat16_as_ushort(v);
+}
+
+// The offsets a look at some rows on the host found, each with the position of
+// one entry on it: the table's first contents.  (From an empty table every
+// thread of the search goes for the same slots at once: 1.3 ms of atomics on
+// 250,000 rows.)
+struct DiaSeed {
+    int32_t count;
+    int32_t off[kDiaMax];
+    int32_t at[kDiaMax];
+};
+
+template <typename V>
+__global__ void dia_seed_kernel(DiaSeed seed, const V* __restrict__ vals, DiaTable* T) {
+    const int s = threadIdx.x;
+    if (s < kDiaSlots) {
+        T->off[s] = s < seed.count ? seed.off[s] : kDiaNoOff;
+        T->val[s] = s < seed.count ? value_bits(vals[seed.at[s]]) : kDiaNoVal;
+    }
+    if (s == 0) {
+        T->overflow = T->disorder = T->varying = 0u;
+        T->pairs = 0ull;
+    }
+}
+
+// Every offset col - row of the matrix into the table (new ones in the order
+// found), whether the columns of each row ascend, and whether the entries of
+// each diagonal are all the same number.  A CTA keeps a copy of the table in
+// shared memory, so global atomics happen once per offset and CTA.
+template <typename V>
+__global__ void __launch_bounds__(kThreads)
+    dia_find_kernel(const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
+                    const V* __restrict__ vals, int32_t nrows, DiaTable* T) {
+    __shared__ volatile int32_t off[kDiaSlots];
+    __shared__ volatile uint64_t val[kDiaSlots];
+    if (threadIdx.x < kDiaSlots) {
+        off[threadIdx.x] = __ldcg(&T->off[threadIdx.x]);
+        val[threadIdx.x] = __ldcg(reinterpret_cast<unsigned long long*>(&T->val[threadIdx.x]));
+    }
+    __syncthreads();
+    bool varying = false;
+    for (int64_t r = int64_t(blockIdx.x) * kThreads + threadIdx.x; r < nrows;
+         r += int64_t(gridDim.x) * kThreads) {
+        if (__ldcg(&T->overflow) | __ldcg(&T->disorder)) return;
+        const int32_t z1 = __ldg(rp + r + 1);
+        int32_t prev = -1;
+        for (int32_t z = __ldg(rp + r); z < z1; ++z) {
+            const int32_t c = __ldg(ci + z);
+            if (c <= prev) {
+                T->disorder = 1u;
+                return;
+            }
+            prev = c;
+            const int32_t d = c - static_cast<int32_t>(r);
+            // its slot: the first that holds it; an empty slot of the copy is
+            // taken (or found taken) in the table, one read of a slot a turn
+            int s = 0;
+            while (s < kDiaSlots) {
+                int32_t have = off[s];
+                if (have == kDiaNoOff) {
+                    const int32_t old = atomicCAS(&T->off[s], kDiaNoOff, d);
+                    have = old == kDiaNoOff ? d : old;
+                    off[s] = have;
+                }
+                if (have == d) break;
+                ++s;
+            }
+            if (s >= kDiaMax) {
+                T->overflow = 1u;
+                return;
+            }
+            if (!varying) {
+                const uint64_t b = value_bits(__ldg(vals + z));
+                uint64_t have = val[s];
+                if (have == kDiaNoVal) {
+                    const unsigned long long old =
+                        atomicCAS(reinterpret_cast<unsigned long long*>(&T->val[s]),
+                                  static_cast<unsigned long long>(kDiaNoVal), b);
+                    have = old == kDiaNoVal ? b : old;
+                    val[s] = have;
+                }
+                varying = have != b || b == kDiaNoVal;
+                if (varying) T->varying = 1u;
+            }
+        }
+    }
+}
+
+struct DiaOffsets {
+    int32_t off[kDiaMax];
+};
+
+// Masks (and, where val is set, values by diagonal) from the CSR arrays; per
+// warp of 32 rows the diagonals it touches are counted into T->pairs.
+template <typename V, typename M>
+__global__ void __launch_bounds__(kThreads)
+    dia_fill_kernel(const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
+                    const V* __restrict__ vals, int32_t nrows, DiaOffsets o, M* __restrict__ mask,
+                    V* __restrict__ val, int64_t ld, DiaTable* T) {
+    const int64_t r = int64_t(blockIdx.x) * kThreads + threadIdx.x;
+    uint32_t m = 0;
+    if (r < nrows) {
+        const int32_t z1 = __ldg(rp + r + 1);
+        int k = 0;  // columns ascend, so do their diagonals
+        for (int32_t z = __ldg(rp + r); z < z1; ++z) {
+            const int32_t d = __ldg(ci + z) - static_cast<int32_t>(r);
+            while (k < kDiaMax - 1 && o.off[k] != d) ++k;
+            m |= 1u << k;
+            if (val) val[int64_t(k) * ld + r] = __ldg(vals + z);
+        }
+        mask[r] = static_cast<M>(m);
+    }
+    const uint32_t any = __reduce_or_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0 && any) atomicAdd(&T->pairs, static_cast<unsigned long long>(__popc(any)));
+}
+
+template <typename V>
+int find_form(nm_csr* A, const DiaSeed& seed) {
+    DiaTable* T = reinterpret_cast<DiaTable*>(A->d_dia_room);
+    const V* vals = static_cast<const V*>(A->d_values);
+    const int32_t n = A->nrows;
+    dia_seed_kernel<V><<<1, 32>>>(seed, vals, T);
+    const int64_t want = (int64_t(n) + kThreads - 1) / kThreads;
+    dia_find_kernel<V><<<static_cast<int>(std::min<int64_t>(want, int64_t(sm_count()) * 8)),
+                         kThreads>>>(A->d_row_ptr, A->d_col_idx, vals, n, T);
+    NM_CHECK_LAUNCH();
+    DiaTable h;
+    NM_CUDA_TRY(cudaMemcpy(&h, T, sizeof h, cudaMemcpyDeviceToHost));
+    if (h.overflow || h.disorder) return NM_OK;
+    int order[kDiaSlots], nd = 0;
+    for (int s = 0; s < kDiaMax; ++s)
+        if (h.off[s] != kDiaNoOff) order[nd++] = s;
+    if (nd == 0) return NM_OK;
+    std::sort(order, order + nd, [&](int a, int b) { return h.off[a] < h.off[b]; });
+    const bool constant = h.varying == 0;
+    if (!constant && 2 * int64_t(A->nnz) < int64_t(nd) * n) return NM_OK;  // mostly padding
+    DiaForm f;
+    f.constant = constant;
+    f.ld = (int64_t(n) + 31) & ~int64_t(31);
+    DiaOffsets o{};
+    for (int k = 0; k < kDiaMax; ++k) {
+        f.off[k] = o.off[k] = k < nd ? h.off[order[k]] : 0;
+        if (k >= nd || !constant) continue;
+        const uint64_t b = h.val[order[k]];
+        if (sizeof(V) == 8) {
+            std::memcpy(&f.cval[k], &b, 8);
+        } else {
+            const uint32_t u = sizeof(V) == 4 ? uint32_t(b) : uint32_t(b) << 16;
+            float x;
+            std::memcpy(&x, &u, 4);
+            f.cval[k] = x;
+        }
+    }
+    f.d_mask = A->d_dia_room + kDiaTableBytes;
+    if (!constant &&
+        cudaMalloc(&f.d_val, sizeof(V) * size_t(nd) * size_t(f.ld)) != cudaSuccess) {
+        cudaGetLastError();  // no room beside the CSR arrays: they serve alone
+        return NM_OK;
+    }
+    if (nd <= 8)
+        dia_fill_kernel<V, uint8_t><<<static_cast<int>(want), kThreads>>>(
+            A->d_row_ptr, A->d_col_idx, vals, n, o, static_cast<uint8_t*>(f.d_mask),
+            static_cast<V*>(f.d_val), f.ld, T);
+    else
+        dia_fill_kernel<V, uint16_t><<<static_cast<int>(want), kThreads>>>(
+            A->d_row_ptr, A->d_col_idx, vals, n, o, static_cast<uint16_t*>(f.d_mask),
+            static_cast<V*>(f.d_val), f.ld, T);
+    cudaError_t e = cudaGetLastError();
+    bool ragged = false;
+    if (constant) {
+        if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // complete for every stream
+    } else {
+        // A warp reads a whole 32-row piece of every diagonal one of its rows
+        // has: rows that share their diagonals read little they do not use.
+        if (e == cudaSuccess) e = cudaMemcpy(&h, T, sizeof h, cudaMemcpyDeviceToHost);
+        ragged = 32 * h.pairs > (unsigned long long)A->nnz * 5 / 4 + 32 * kDiaMax;
+    }
+    if (e != cudaSuccess || ragged) {
+        if (f.d_val) cudaFree(f.d_val);
+        NM_CUDA_TRY(e);
+        return NM_OK;
+    }
+    f.ndiag = nd;
+    A->dia = f;
+    return NM_OK;
+}
+
+// ---------------------------------------------------------------------------
+// y = A x.  kDiaR rows per thread and step, a persistent grid; the masks of
+// the next step are loaded under this step's products.  A warp whose rows all
+// have every diagonal takes a path without predicates.  Offsets and constant
+// values sit in registers: as kernel-parameter operands they cost a load per
+// use (118 against 50 instructions per warp of rows).
+// ---------------------------------------------------------------------------
+constexpr int kDiaThreads = 128;
+
+template <typename V, typename X, typename A, int KC, bool CONST, int R>
+__global__ void __launch_bounds__(kDiaThreads)
+    spmv_dia_kernel(const DiaView<A> D, int ndiag, const X* __restrict__ x, X* __restrict__ y) {
+    using M = DiaMask<KC>;
+    const M* __restrict__ mask = static_cast<const M*>(D.mask);
+    const V* __restrict__ val = static_cast<const V*>(D.val);
+    const uint32_t full_mask = (1u << ndiag) - 1u;
+    const int64_t n = D.n, step = int64_t(gridDim.x) * (kDiaThreads * R);
+    int32_t off[KC];
+    A cv[KC];
+#pragma unroll
+    for (int k = 0; k < KC; ++k) {
+        off[k] = D.off[k];
+        asm volatile("" : "+r"(off[k]));
+        cv[k] = D.cval[k];
+        if constexpr (CONST && sizeof(A) == 8) asm volatile("" : "+d"(cv[k]));
+        if constexpr (CONST && sizeof(A) == 4) asm volatile("" : "+f"(cv[k]));
+    }
+    int64_t b = int64_t(blockIdx.x) * (kDiaThreads * R) + threadIdx.x;
+    uint32_t m[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) m[r] = b + r * kDiaThreads < n ? mask[b + r * kDiaThreads] : 0u;
+    for (; b - int(threadIdx.x) < n; b += step) {
+        const X* xp[KC];
+#pragma unroll
+        for (int k = 0; k < KC; ++k) xp[k] = x + (b + off[k]);
+        A xs[R][KC], vs[R][KC];
+        bool full[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            full[r] = KC == ndiag && __all_sync(0xffffffffu, m[r] == full_mask);
+            const V* vp = val + (b + r * kDiaThreads);
+            if (full[r]) {
+#pragma unroll
+                for (int k = 0; k < KC; ++k) {
+                    xs[r][k] = static_cast<A>(__ldg(xp[k] + r * kDiaThreads));
+                    vs[r][k] = CONST ? cv[k] : widen<V, A>(ld_value_cs(vp + k * D.ld));
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < KC; ++k) {
+                    xs[r][k] = A(0);
+                    vs[r][k] = cv[k];
+                    if (m[r] >> k & 1u) {
+                        xs[r][k] = static_cast<A>(__ldg(xp[k] + r * kDiaThreads));
+                        if constexpr (!CONST) vs[r][k] = widen<V, A>(ld_value_cs(vp + k * D.ld));
+                    }
+                }
+            }
+        }
+        uint32_t mn[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int64_t nx = b + step + r * kDiaThreads;
+            mn[r] = nx < n ? mask[nx] : 0u;
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            A acc = A(0);
+            const int64_t row = b + r * kDiaThreads;
+            if (full[r]) {
+#pragma unroll
+                for (int k = 0; k < KC; ++k) acc = add_rn(acc, mul_rn(vs[r][k], xs[r][k]));
+                y[row] = static_cast<X>(acc);
+            } else {
+#pragma unroll
+                for (int k = 0; k < KC; ++k)
+                    if (m[r] >> k & 1u) acc = add_rn(acc, mul_rn(vs[r][k], xs[r][k]));
+                if (row < n) y[row] = static_cast<X>(acc);
+            }
+            m[r] = mn[r];
+        }
+    }
+}
+
+template <typename V, typename X, typename A, int KC, bool CONST, int R>
+int launch_dia_r(const nm_csr* M, const X* x, X* y, cudaStream_t s) {
+    int occ = 0;
+    const auto fn = spmv_dia_kernel<V, X, A, KC, CONST, R>;
+    const int st = kernel_occupancy(reinterpret_cast<const void*>(fn), kDiaThreads, &occ);
+    if (st != NM_OK) return st;
+    const int64_t need = (int64_t(M->nrows) + kDiaThreads * R - 1) / (kDiaThreads * R);
+    const int grid = static_cast<int>(std::min<int64_t>(need, int64_t(sm_count()) * occ));
+    fn<<<grid, kDiaThreads, 0, s>>>(dia_view<A>(M->dia, M->nrows), M->dia.ndiag, x, y);
+    NM_CHECK_LAUNCH();
+    return NM_OK;
+}
+
+// One row per thread while the rows fit the resident threads at one each (no
+// thread then waits for a second row's loads), else two.
+template <typename V, typename X, typename A, int KC>
+int launch_dia_k(const nm_csr* M, const X* x, X* y, cudaStream_t s) {
+    const bool one = int64_t(M->nrows) <= int64_t(sm_count()) * 1024;
+    if (M->dia.constant)
+        return one ? launch_dia_r<V, X, A, KC, true, 1>(M, x, y, s)
+                   : launch_dia_r<V, X, A, KC, true, 2>(M, x, y, s);
+    return one ? launch_dia_r<V, X, A, KC, false, 1>(M, x, y, s)
+               : launch_dia_r<V, X, A, KC, false, 2>(M, x, y, s);
+}
+
+template <typename V, typename X, typename A>
+int launch_dia_t(const nm_csr* M, const void* x, void* y, cudaStream_t s) {
+    const X* xx = static_cast<const X*>(x);
+    X* yy = static_cast<X*>(y);
+    const int nd = M->dia.ndiag;
+    if (nd <= 3) return launch_dia_k<V, X, A, 3>(M, xx, yy, s);
+    if (nd <= 5) return launch_dia_k<V, X, A, 5>(M, xx, yy, s);
+    if (nd <= 7) return launch_dia_k<V, X, A, 7>(M, xx, yy, s);
+    if (nd <= 8) return launch_dia_k<V, X, A, 8>(M, xx, yy, s);
+    if (nd <= 9) return launch_dia_k<V, X, A, 9>(M, xx, yy, s);  // 16-bit masks from here on
+    return launch_dia_k<V, X, A, kDiaMax>(M, xx, yy, s);
+}
+
+}  // namespace
+
+int find_dia_form(nm_csr* A) {
+    if (A->nnz == 0 || A->nrows == 0) return NM_OK;
+    // A look at some rows on the host first: a matrix of scattered columns
+    // shows more than kDiaMax offsets there and costs nothing more.
+    const int32_t* rp = A->h_row_ptr.data();
+    const int32_t* ci = A->h_col_idx.data();
+    DiaSeed seed{};
+    constexpr int kLook = 64;
+    for (int q = 0; q < kLook; ++q) {
+        const int32_t r = static_cast<int32_t>(int64_t(A->nrows - 1) * q / (kLook - 1));
+        if (rp[r + 1] - rp[r] > kDiaMax) return NM_OK;
+        for (int32_t z = rp[r]; z < rp[r + 1]; ++z) {
+            const int32_t d = ci[z] - r;
+            if (std::find(seed.off, seed.off + seed.count, d) != seed.off + seed.count) continue;
+            if (seed.count == kDiaMax) return NM_OK;
+            seed.off[seed.count] = d;
+            seed.at[seed.count++] = z;
+        }
+    }
+    switch (A->dtype) {
+        case NM_F64: return find_form<double>(A, seed);
+        case NM_F32: return find_form<float>(A, seed);
+        default: return find_form<__nv_bfloat16>(A, seed);
+    }
+}
+
+int launch_spmv_dia(const nm_csr* A, const void* x, void* y, cudaStream_t s) {
+    switch (A->dtype) {
+        case NM_F64: return launch_dia_t<double, double, double>(A, x, y, s);
+        case NM_F32: return launch_dia_t<float, float, float>(A, x, y, s);
+        default: return launch_dia_t<__nv_bfloat16, float, float>(A, x, y, s);
+    }
+}
+
+}  // namespace nm

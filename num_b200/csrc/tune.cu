@@ -6,8 +6,8 @@
 //   short_max 32, 64             rows up to this length are thread-per-row
 //   stages    2, 3, 4            TMA ring depth (skipped when it does not fit)
 //   grid_mult 0 (all resident CTAs), 1, 2 CTAs per SM
-//   and, once each, the warp-gather and sliced gather kernels (which ignore
-//   the four above)
+//   and, once each, the warp-gather and sliced gather kernels and, where the
+//   matrix has one, its diagonal form under AUTO (which ignore the four above)
 // max_rows stays at its default (one consumer thread per row of a block).
 // tile and short_max change the descriptors (a host rebuild per pair);
 // stages and grid_mult only change the launch.  short_max never goes below
@@ -133,6 +133,27 @@ extern "C" int nm_csr_autotune(nm_csr* A, const void* x, void* y, void* stream,
                 win = A->tune;
                 win_us = us;
                 have = true;
+            }
+        }
+    }
+    if (st == NM_OK && A->dia.ndiag > 0) {
+        // the diagonal form, which only AUTO runs
+        nm_tuning t = start;
+        t.short_max = kDefaultShortMax;
+        t.kernel = NM_KERNEL_AUTO;
+        A->tune = t;
+        st = rebuild_blocks(A);
+        float us = 0.f;
+        if (st == NM_OK && A->use_dia()) {
+            st = time_spmv(A, x, y, s, 1, reps, ev.a, ev.b, &us);
+            if (st == NM_OK) {
+                if (n < cap) trials[n] = nm_tune_trial{A->tune, us};
+                ++n;
+                if (!have || us < win_us) {
+                    win = A->tune;
+                    win_us = us;
+                    have = true;
+                }
             }
         }
     }

@@ -425,8 +425,9 @@ def tuning(A: CrsMatrix) -> dict:
 
 
 def spmv_kernel(A: CrsMatrix) -> str:
-    """The kernel spmv runs on A: "blocks" (row-block pipeline) or "gather"
-    (warp per 32 rows, for scattered columns)."""
+    """The kernel spmv runs on A: "blocks" (row-block pipeline, also its
+    diagonal form under "auto") or "gather" (warp per 32 rows, for scattered
+    columns)."""
     k = C.c_int32()
     _lib.check(_lib.load().nm_csr_spmv_kernel(A._h, C.byref(k)))
     return {v: n for n, v in _KERNELS.items()}[k.value]
