@@ -812,7 +812,7 @@ def run_cg(args, rank, world, local_rank):
                 "api": "kokkos_spmv.cg_solve_local with pinned b copied in and x copied out"},
         # per solve: A x0, the initial kernel, then one persistent launch, or
         # two kernels per iteration on the CUDA-graph path
-        "gpu_launches": int(3 * args.steps if r["path_id"] in (1, 2, 3, 4)
+        "gpu_launches": int(3 * args.steps if r["path_id"] in (1, 2, 3, 4, 5)
                             else r["iters"] * 2 + 2 * args.steps),
         "clocks": r["clocks"],
     })

@@ -244,8 +244,12 @@ int nm_scale(int64_t n, double alpha, double* x, void* stream);
 /* ---- CG -------------------------------------------------------------------- */
 
 /* Process-wide choice of how nm_cg_local / nm_dist_cg_single iterate:
- * 1 (default) one persistent launch per solve for systems of at most 262,144
- * rows -- the cluster solve where it applies (systems of at most 65,536 rows
+ * 1 (default) one persistent launch per solve for matrices of more than 32,768
+ * rows on at most 8 diagonals, up to 1,060,864 rows (262,144 where the values
+ * on a diagonal vary), and for other systems of at most 262,144 rows -- the
+ * solve on the diagonal form for the first (x, r and the direction on chip over
+ * all SMs, two all-to-all exchanges of sums per iteration), for the others the
+ * cluster solve where it applies (systems of at most 65,536 rows
  * of at most 8 nonzeros on one 16-CTA thread-block cluster: the rows of A in
  * shared memory, each CTA's halo of the direction kept current over
  * distributed shared memory, two hardware cluster barriers per iteration),
@@ -257,7 +261,9 @@ int nm_scale(int64_t n, double alpha, double* x, void* stream);
  * iteration, the SpMV forming p = r + beta p as it reads it (also what 2 to 4
  * run where their path does not apply).  All
  * give the same iterates, bit for bit (every dot product is summed in one
- * fixed order: per row block or 256-row tile, then over the blocks).  Other
+ * fixed order: per row block or 256-row tile, then over the blocks), but that
+ * above 262,144 rows the solve on the diagonal form and the graph each have
+ * their own.  Other
  * values: NM_ERR_INVALID.  No reference counterpart (an implementation
  * switch). */
 int nm_cg_set_persistent(int32_t enable);
@@ -265,7 +271,8 @@ int nm_cg_set_persistent(int32_t enable);
 /* How the last nm_cg_local / nm_dist_cg_single solve on A iterated: 0 the
  * CUDA-graph chunks, 1 the TMA-pipelined persistent solve (three grid
  * barriers per iteration), 2 the same in its two-barrier form, 3 the resident
- * solve, 4 the cluster solve; -1 before A's first solve.  No reference
+ * solve, 4 the cluster solve, 5 the solve on the diagonal form; -1 before A's
+ * first solve.  No reference
  * counterpart. */
 int nm_cg_last_path(const nm_csr* A, int32_t* path);
 

@@ -517,6 +517,7 @@ CgWorkspace::~CgWorkspace() {
     cudaFree(dmem);
     if (res_mem) cudaFree(res_mem);
     if (cl_mem) cudaFree(cl_mem);
+    if (dia_mem) cudaFree(dia_mem);
     pinned_slots().put(h_in);
     pinned_slots().put(h_out);
 }
@@ -646,12 +647,11 @@ int ensure_workspace(nm_csr* A, CgWorkspace** out) {
         const bool fits = coop_ok && n <= kCoopMaxRows;
         ws->coop_formed = fits && int64_t(occ_f) * sm_count() >= ws->grid_spmv;
         ws->coop = ws->coop_formed || (fits && int64_t(occ_c) * sm_count() >= ws->grid_spmv);
+        ws->coop_launch = coop_ok != 0;
         if (coop_ok) {
-            st = plan_resident(A, ws.get());
+            st = plan_dia(A, ws.get());
             if (st != NM_OK) return st;
         }
-        st = plan_cluster(A, ws.get());
-        if (st != NM_OK) return st;
     }
     ws->err = device_error_word();
     if (!ws->err) return fail(NM_ERR_CUDA, "cg: cannot map the device error word");
@@ -793,19 +793,34 @@ int cg_run(nm_csr* A, const double* b, double* x, double tol, int32_t max_iter, 
     NM_CHECK_LAUNCH();
 
     const int mode = g_cg_persistent.load();
-    // mode 1: the cluster solve where it applies (6.0 us per iteration on the
-    // 256^2 Laplacian), else the TMA-pipelined persistent solve where it fits
-    // (9.8 us there), else the resident one (10.8 us); 2, 3, 4: the second,
-    // the third, the first only; 0: graph chunks
-    const bool cluster = ws->cluster && (mode == 4 || mode == 1);
-    const bool resident = !cluster && ws->resident && (mode == 3 || (mode == 1 && !ws->coop));
-    const bool coop = cluster || resident || (ws->coop && (mode == 1 || mode == 2));
+    // mode 1: the solve on the diagonal form where it applies (4.5 us per
+    // iteration on the 256^2 Laplacian), else the cluster solve (6.0 us there),
+    // else the TMA-pipelined persistent solve where it fits (9.8 us), else the
+    // resident one (10.8 us); 2, 3, 4: the pipelined, the resident, the cluster
+    // solve only; 0: graph chunks
+    const bool dia = ws->dia && mode == 1;
+    // (the cluster and resident solves are planned when first in question)
+    if (!dia && (mode == 4 || mode == 1) && !ws->cluster_planned) {
+        st = plan_cluster(A, ws);
+        if (st != NM_OK) return st;
+        ws->cluster_planned = true;
+    }
+    const bool cluster = !dia && ws->cluster && (mode == 4 || mode == 1);
+    const bool want_resident = !dia && !cluster && (mode == 3 || (mode == 1 && !ws->coop));
+    if (want_resident && ws->coop_launch && !ws->resident_planned) {
+        st = plan_resident(A, ws);
+        if (st != NM_OK) return st;
+        ws->resident_planned = true;
+    }
+    const bool resident = want_resident && ws->resident;
+    const bool coop = dia || cluster || resident || (ws->coop && (mode == 1 || mode == 2));
     if (coop) {
         // the whole iteration loop in one persistent launch
-        st = cluster ? launch_cluster(A, ws, s)
-                     : (resident ? launch_resident(A, ws, s) : launch_coop(A, ws, s));
+        st = dia ? launch_dia_cg(A, ws, s)
+             : cluster ? launch_cluster(A, ws, s)
+                       : (resident ? launch_resident(A, ws, s) : launch_coop(A, ws, s));
         if (st != NM_OK) return st;
-        ws->last_path = cluster ? 4 : (resident ? 3 : (ws->coop_formed ? 2 : 1));
+        ws->last_path = dia ? 5 : (cluster ? 4 : (resident ? 3 : (ws->coop_formed ? 2 : 1)));
         NM_CUDA_TRY(cudaMemcpyAsync(ws->h_out, ws->st, sizeof(CgState), cudaMemcpyDeviceToHost, s));
         NM_CUDA_TRY(cudaStreamSynchronize(s));
     }

@@ -50,6 +50,8 @@ struct CgWorkspace {
     unsigned int* err = nullptr;  // device error word (not owned)
     cudaStream_t cap_stream = nullptr;
     std::map<int, cudaGraphExec_t> graphs;  // iterations per graph -> exec
+    bool coop_launch = false;  // the device takes cooperative launches
+    bool resident_planned = false, cluster_planned = false;
     // the resident solve (cg_resident.cu), when the matrix qualifies
     bool resident = false;
     int32_t last_path = -1;  // path of the last solve (nm_cg_last_path)
@@ -67,8 +69,23 @@ struct CgWorkspace {
     uint16_t* cl_lcol = nullptr;
     int32_t* cl_push_off = nullptr;
     uint32_t* cl_push_ent = nullptr;
+    // the solve on the diagonal form (cg_dia.cu), when the matrix has one
+    bool dia = false, dia_tiles = false;  // dia_tiles: sums per tile, else per CTA
+    int dia_q = 0, dia_b = 0, dia_grid = 0;  // rows per thread, tiles per CTA, CTAs
+    bool dia_early = false;  // room in shared memory for other CTAs' r
+    size_t dia_smem = 0;
+    void* dia_mem = nullptr;  // the words of r and of the sums
     ~CgWorkspace();
 };
+
+// The solve on the diagonal form: matrices of more than 32,768 rows on at most
+// 8 diagonals whose row blocks are whole 256-row tiles, up to 14 rows per
+// thread of one 512-thread CTA per SM (1,060,864 rows on 148 SMs; 262,144 when
+// the values on a diagonal vary).  NM_OK with ws->dia false when A does not
+// qualify.
+int plan_dia(const nm_csr* A, CgWorkspace* ws);
+// One such solve on `s` after cg_init_kernel (ws->r, ws->p hold r0 = p0).
+int launch_dia_cg(const nm_csr* A, CgWorkspace* ws, cudaStream_t s);
 
 // The cluster solve: systems whose row blocks are whole 256-row tiles and
 // whose rows fit the cluster's shared memory -- when every value is a float
@@ -125,6 +142,31 @@ __device__ __forceinline__ bool grid_reduce_last(const double (&part)[K], double
     }
     if (threadIdx.x == 0) *counter = 0u;
     return threadIdx.x == 0;
+}
+
+// The warp sums of P values per lane at once (P a power of two <= 8): the
+// same pairing as warp_sum's shuffle tree, value by value -- stage o adds the
+// partials of lanes l and l ^ o -- but at each of the first log2(P) stages a
+// lane keeps half of its values and hands the partner the other half, so the
+// P trees take P - 1 + 5 - log2(P) shuffles instead of 5 P.  Afterwards v[0]
+// of lane l holds the sum of value (l >> (5 - log2 P)) & (P - 1).
+template <int P>
+__device__ __forceinline__ void multi_warp_sum(double (&v)[P]) {
+    const int lane = threadIdx.x & 31;
+    int o = 16;
+#pragma unroll
+    for (int cnt = P; cnt > 1; cnt >>= 1, o >>= 1) {
+        const bool hi = (lane & o) != 0;
+        const int half = cnt >> 1;
+#pragma unroll
+        for (int j = 0; j < half; ++j) {
+            const double send = hi ? v[j] : v[j + half];
+            const double keep = hi ? v[j + half] : v[j];
+            v[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+#pragma unroll
+    for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
 }
 
 // Sum over the first 8 warps (256 threads) of the CTA: a shuffle tree per warp,

@@ -92,31 +92,6 @@ struct ClusterArgs {
     int32_t pmax;   // push entries of the CTA with the most
 };
 
-// The warp sums of P values per lane at once (P a power of two <= 8): the
-// same pairing as warp_sum's shuffle tree, value by value -- stage o adds the
-// partials of lanes l and l ^ o -- but at each of the first log2(P) stages a
-// lane keeps half of its values and hands the partner the other half, so the
-// P trees take P - 1 + 5 - log2(P) shuffles instead of 5 P.  Afterwards v[0]
-// of lane l holds the sum of value (l >> (5 - log2 P)) & (P - 1).
-template <int P>
-__device__ __forceinline__ void multi_warp_sum(double (&v)[P]) {
-    const int lane = threadIdx.x & 31;
-    int o = 16;
-#pragma unroll
-    for (int cnt = P; cnt > 1; cnt >>= 1, o >>= 1) {
-        const bool hi = (lane & o) != 0;
-        const int half = cnt >> 1;
-#pragma unroll
-        for (int j = 0; j < half; ++j) {
-            const double send = hi ? v[j] : v[j + half];
-            const double keep = hi ? v[j + half] : v[j];
-            v[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-        }
-    }
-#pragma unroll
-    for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
-}
-
 constexpr int pow2_at_least(int r) { return r <= 1 ? 1 : (r <= 2 ? 2 : (r <= 4 ? 4 : 8)); }
 constexpr int log2_of(int p) { return p <= 1 ? 0 : 1 + log2_of(p / 2); }
 
