@@ -203,6 +203,10 @@ int build_sell(nm_csr* A);
 int find_dia_form(nm_csr* A);
 // y = A x on the diagonal form.
 int launch_spmv_dia(const nm_csr* A, const void* x, void* y, cudaStream_t stream);
+// Y = A X (row-major, k columns; vec2: k even and X, Y 16-byte aligned) on the
+// diagonal form.
+int launch_batch_dia(const nm_csr* A, const double* X, double* Y, int32_t k, bool vec2,
+                     cudaStream_t stream);
 // Drops A's cached CG workspace (its graphs hold the current descriptors).
 void reset_cg(nm_csr* A);
 // Nonzeros of the Laplacian on an L^dim grid (dim 2: 5-point, dim 3: 7-point).

@@ -339,6 +339,204 @@ int launch_dia_t(const nm_csr* M, const void* x, void* y, cudaStream_t s) {
     return launch_dia_k<V, X, A, kDiaMax>(M, xx, yy, s);
 }
 
+// ---------------------------------------------------------------------------
+// Y = A X for k right-hand sides (row-major).  A CTA walks a run of
+// consecutive rows, for a chunk of at most 16 columns; a row's columns of the
+// chunk lie on 2^lg consecutive lanes, VEC to a lane.  Walking in row order,
+// the CTA finds the rows of X that its near diagonals share in L1: 128 bytes a
+// row, and at each step only the outermost diagonals bring new ones.  (One
+// warp per row over all columns, rows strided over the GPU, reads 5.5 rows of
+// X from L2 per row on a 7-point stencil; this reads 3.2.)  The chunks of a
+// run are neighbouring CTAs, so that whole rows of X come from HBM once.
+// ---------------------------------------------------------------------------
+//
+// 100^3, k = 128 (2.14 GB): 431 us against 650 us; k = 33: 191 against 454;
+// 500^2, k = 17: 29 against 109.  32-column chunks 537 us, 8-column 555;
+// CTAs of 256 threads on 512-row runs 455 us, of 512 threads 484; 96- and
+// 320-row runs 442 and 473 us.  What is left waits on X
+// from L2: registers allow 28 of 64 warps per SM, and L1 holds 36 % of the
+// loads.
+constexpr int kDiaBatchThreads = 128;
+constexpr int kDiaBatchCols = 16;
+constexpr int kDiaBatchRun = 192;
+
+template <int KC, bool CONST, int VEC>
+__global__ void __launch_bounds__(kDiaBatchThreads)
+    batch_dia_kernel(const DiaView<double> D, int ndiag, int32_t k, int lg, int chunk_cols, int nchunk,
+                     int32_t run, const double* __restrict__ X, double* __restrict__ Y) {
+    using M = DiaMask<KC>;
+    const M* __restrict__ mask = static_cast<const M*>(D.mask);
+    const double* __restrict__ val = static_cast<const double*>(D.val);
+    const int chunk = blockIdx.x % nchunk;
+    const int64_t r_begin = int64_t(blockIdx.x / nchunk) * run;
+    const int64_t r_end = min(int64_t(D.n), r_begin + run);
+    const int c = chunk * chunk_cols + (threadIdx.x & ((1 << lg) - 1)) * VEC;
+    const bool in = c < min(k, (chunk + 1) * chunk_cols);
+    const int step = kDiaBatchThreads >> lg;
+    // Distances to the diagonals' rows of X and their values in registers.
+    int64_t dist[KC];
+    double cv[KC];
+#pragma unroll
+    for (int e = 0; e < KC; ++e) {
+        dist[e] = int64_t(D.off[e]) * k;
+        cv[e] = D.cval[e];
+        asm volatile("" : "+l"(dist[e]));
+        if constexpr (CONST) asm volatile("" : "+d"(cv[e]));
+    }
+    const uint32_t full_mask = (1u << ndiag) - 1u;
+    int64_t row = r_begin + (threadIdx.x >> lg);
+    const double* xp = X + row * k + c;
+    double* yp = Y + row * k + c;
+    const int64_t adv = int64_t(step) * k;
+    uint32_t m = row < r_end && in ? mask[row] : 0u;
+    for (; row - (threadIdx.x >> lg) < r_end; row += step, xp += adv, yp += adv) {
+        double x[KC][VEC], v[KC];
+        const uint32_t mc = m;
+        const bool full = KC == ndiag && __all_sync(0xffffffffu, mc == full_mask);
+        auto load = [&](int e) {
+            if constexpr (VEC == 2) {
+                const double2 t = __ldg(reinterpret_cast<const double2*>(xp + dist[e]));
+                x[e][0] = t.x;
+                x[e][1] = t.y;
+            } else {
+                x[e][0] = __ldg(xp + dist[e]);
+            }
+            v[e] = CONST ? cv[e] : __ldg(val + e * D.ld + row);
+        };
+        if (full) {
+#pragma unroll
+            for (int e = 0; e < KC; ++e) load(e);
+        } else {
+#pragma unroll
+            for (int e = 0; e < KC; ++e)
+                if (mc >> e & 1u) load(e);
+        }
+        m = row + step < r_end && in ? mask[row + step] : 0u;
+        double acc[VEC];
+#pragma unroll
+        for (int q = 0; q < VEC; ++q) acc[q] = 0.0;
+        if (full) {
+#pragma unroll
+            for (int e = 0; e < KC; ++e)
+#pragma unroll
+                for (int q = 0; q < VEC; ++q) acc[q] = add_rn(acc[q], mul_rn(v[e], x[e][q]));
+        } else {
+#pragma unroll
+            for (int e = 0; e < KC; ++e)
+                if (mc >> e & 1u) {
+#pragma unroll
+                    for (int q = 0; q < VEC; ++q) acc[q] = add_rn(acc[q], mul_rn(v[e], x[e][q]));
+                }
+        }
+        if (in && row < r_end) {
+            if constexpr (VEC == 2) *reinterpret_cast<double2*>(yp) = make_double2(acc[0], acc[1]);
+            else yp[0] = acc[0];
+        }
+    }
+}
+
+// The same for more than 8 diagonals: rows of a matrix with that many use few
+// of them (a periodic grid's wrap-around diagonals), so a row's diagonals are
+// taken from its mask, kDiaBits at a time, instead of asking each in turn.
+constexpr int kDiaBits = 6;
+
+template <bool CONST, int VEC>
+__global__ void __launch_bounds__(kDiaBatchThreads)
+    batch_dia_bits_kernel(const DiaView<double> D, int32_t k, int lg, int chunk_cols, int nchunk,
+                          int32_t run, const double* __restrict__ X, double* __restrict__ Y) {
+    __shared__ int64_t dist[kDiaMax];  // to the diagonal's row of X
+    __shared__ double cv[kDiaMax];
+    if (threadIdx.x < kDiaMax) {
+        dist[threadIdx.x] = int64_t(D.off[threadIdx.x]) * k;
+        cv[threadIdx.x] = D.cval[threadIdx.x];
+    }
+    __syncthreads();
+    const uint16_t* __restrict__ mask = static_cast<const uint16_t*>(D.mask);
+    const double* __restrict__ val = static_cast<const double*>(D.val);
+    const int chunk = blockIdx.x % nchunk;
+    const int64_t r_begin = int64_t(blockIdx.x / nchunk) * run;
+    const int64_t r_end = min(int64_t(D.n), r_begin + run);
+    const int c = chunk * chunk_cols + (threadIdx.x & ((1 << lg) - 1)) * VEC;
+    if (c >= min(k, (chunk + 1) * chunk_cols)) return;
+    const int step = kDiaBatchThreads >> lg;
+    int64_t row = r_begin + (threadIdx.x >> lg);
+    uint32_t m = row < r_end ? mask[row] : 0u;
+    for (; row < r_end; row += step) {
+        uint32_t left = m;
+        m = row + step < r_end ? mask[row + step] : 0u;
+        const double* xp = X + row * k + c;
+        double acc[VEC];
+#pragma unroll
+        for (int q = 0; q < VEC; ++q) acc[q] = 0.0;
+        while (left) {
+            double x[kDiaBits][VEC], v[kDiaBits];
+            const int cnt = __popc(left);
+#pragma unroll
+            for (int j = 0; j < kDiaBits; ++j)
+                if (j < cnt) {
+                    const int e = __ffs(left) - 1;
+                    left &= left - 1u;
+                    if constexpr (VEC == 2) {
+                        const double2 t = __ldg(reinterpret_cast<const double2*>(xp + dist[e]));
+                        x[j][0] = t.x;
+                        x[j][1] = t.y;
+                    } else {
+                        x[j][0] = __ldg(xp + dist[e]);
+                    }
+                    v[j] = CONST ? cv[e] : __ldg(val + e * D.ld + row);
+                }
+#pragma unroll
+            for (int j = 0; j < kDiaBits; ++j)
+                if (j < cnt) {
+#pragma unroll
+                    for (int q = 0; q < VEC; ++q) acc[q] = add_rn(acc[q], mul_rn(v[j], x[j][q]));
+                }
+        }
+        double* yp = Y + row * k + c;
+        if constexpr (VEC == 2) *reinterpret_cast<double2*>(yp) = make_double2(acc[0], acc[1]);
+        else yp[0] = acc[0];
+    }
+}
+
+template <int KC, bool CONST, int VEC>
+void launch_batch_dia_t(const nm_csr* A, const double* X, double* Y, int32_t k, cudaStream_t s) {
+    // lanes per row: 16 columns to a chunk, or 8 where that leaves fewer
+    // lanes idle in the last one
+    const int groups = (k + VEC - 1) / VEC;
+    int lg = 0;
+    while ((1 << lg) < groups && (VEC << lg) < kDiaBatchCols) ++lg;
+    auto slots = [&](int l) { return ((groups + (1 << l) - 1) >> l) << l; };
+    if ((1 << lg) < groups && lg > 0 && slots(lg - 1) < slots(lg)) --lg;
+    const int nchunk = (groups + (1 << lg) - 1) >> lg;
+    const int chunk_cols = VEC * ((groups + nchunk - 1) / nchunk);
+    const int step = kDiaBatchThreads >> lg;
+    // Shorter runs where there are too few rows to fill the GPU with them.
+    int64_t run = std::max<int64_t>(step, int64_t(A->nrows) * nchunk / (int64_t(sm_count()) * 16));
+    run = (std::min<int64_t>(run, kDiaBatchRun) + step - 1) / step * step;
+    const int64_t grid = (int64_t(A->nrows) + run - 1) / run * nchunk;
+    const auto D = dia_view<double>(A->dia, A->nrows);
+    const unsigned g = static_cast<unsigned>(grid);
+    const int32_t r = static_cast<int32_t>(run);
+    if constexpr (KC > 8)
+        batch_dia_bits_kernel<CONST, VEC><<<g, kDiaBatchThreads, 0, s>>>(D, k, lg, chunk_cols,
+                                                                         nchunk, r, X, Y);
+    else
+        batch_dia_kernel<KC, CONST, VEC><<<g, kDiaBatchThreads, 0, s>>>(
+            D, A->dia.ndiag, k, lg, chunk_cols, nchunk, r, X, Y);
+}
+
+template <int KC>
+void launch_batch_dia_k(const nm_csr* A, const double* X, double* Y, int32_t k, bool vec2,
+                        cudaStream_t s) {
+    if (A->dia.constant) {
+        if (vec2) launch_batch_dia_t<KC, true, 2>(A, X, Y, k, s);
+        else launch_batch_dia_t<KC, true, 1>(A, X, Y, k, s);
+    } else {
+        if (vec2) launch_batch_dia_t<KC, false, 2>(A, X, Y, k, s);
+        else launch_batch_dia_t<KC, false, 1>(A, X, Y, k, s);
+    }
+}
+
 }  // namespace
 
 int find_dia_form(nm_csr* A) {
@@ -373,6 +571,18 @@ int launch_spmv_dia(const nm_csr* A, const void* x, void* y, cudaStream_t s) {
         case NM_F32: return launch_dia_t<float, float, float>(A, x, y, s);
         default: return launch_dia_t<__nv_bfloat16, float, float>(A, x, y, s);
     }
+}
+
+int launch_batch_dia(const nm_csr* A, const double* X, double* Y, int32_t k, bool vec2,
+                     cudaStream_t s) {
+    const int nd = A->dia.ndiag;
+    if (nd <= 3) launch_batch_dia_k<3>(A, X, Y, k, vec2, s);
+    else if (nd <= 5) launch_batch_dia_k<5>(A, X, Y, k, vec2, s);
+    else if (nd <= 7) launch_batch_dia_k<7>(A, X, Y, k, vec2, s);
+    else if (nd <= 8) launch_batch_dia_k<8>(A, X, Y, k, vec2, s);
+    else launch_batch_dia_k<kDiaMax>(A, X, Y, k, vec2, s);
+    NM_CHECK_LAUNCH();
+    return NM_OK;
 }
 
 }  // namespace nm

@@ -726,6 +726,9 @@ static void launch_batch_v(const nm_csr* A, const double* X, double* Y, int32_t 
 static int launch_batch(const nm_csr* A, const double* X, double* Y, int32_t k, cudaStream_t s) {
     const bool vec2 = (k % 2 == 0) && (reinterpret_cast<uintptr_t>(X) % 16 == 0) &&
                       (reinterpret_cast<uintptr_t>(Y) % 16 == 0);
+    // Matrices in diagonal form have kernels of their own (dia.cu); like those
+    // below they sum every (row, column) serially in CSR order.
+    if (A->dia.ndiag > 0) return launch_batch_dia(A, X, Y, k, vec2, s);
     const int vec = vec2 ? 2 : 1;
     const int groups = (k + vec - 1) / vec;  // lane-columns needed for one pass
     int tpr_log2 = 0;

@@ -106,3 +106,22 @@ def test_diagonal_form_of_an_assembled_laplacian(kspmv, oracle):
     y = torch.empty(A.nrows, dtype=torch.float64, device="cuda")
     kspmv.spmv(M, torch.from_numpy(x).cuda(), y)
     assert np.array_equal(y.cpu().numpy(), oracle.spmv(A.row_ptr, A.col_idx, A.values, x))
+
+
+# chunks of one and several lanes, ragged last chunks, 16-byte loads or not,
+# the widest masks, one run and many
+@pytest.mark.parametrize("k", [1, 2, 3, 7, 16, 17, 33, 34, 130])
+@pytest.mark.parametrize("name", ["lap2d_1", "lap2d_33", "lap3d_17", "varcoef_19", "gauge_40",
+                                  "wide", "tall", "eight", "const_9", "diag_129"])
+def test_diagonal_form_multi_rhs_bit_exact(kspmv, oracle, name, k):
+    A = _case(name)
+    X = np.random.default_rng(k).standard_normal((A.ncols, k))
+    M = kspmv.upload_csr(A.row_ptr, A.col_idx, A.values, A.nrows, A.ncols)
+    ref = oracle.batch_spmv(A.row_ptr, A.col_idx, A.values, X)
+    for offset in (0, 1):  # X on a 16-byte boundary, and 8 bytes off it
+        buf = torch.full((A.ncols * k + 1,), float("nan"), dtype=torch.float64, device="cuda")
+        Xd = buf[offset:offset + A.ncols * k].view(A.ncols, k)
+        Xd.copy_(torch.from_numpy(X))
+        Y = torch.full((A.nrows, k), float("nan"), dtype=torch.float64, device="cuda")
+        kspmv.batch_spmv(M, Xd, Y)
+        assert np.array_equal(Y.cpu().numpy(), ref), offset
