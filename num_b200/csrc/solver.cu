@@ -66,17 +66,29 @@ struct SysState {
     double rz_keep;     // r.z of the last completed iteration of the previous inner solve
     double gamma;       // p = z + gamma p at an inner start (0: fresh start)
     unsigned int tile_arrivals;  // large systems: tile CTAs of bs_update done this iteration
-    unsigned int pad2_;
+    unsigned int blk_arrivals;   // ... row blocks of bs_spmv_dia
 };
 
 struct SysRef {
     int32_t slot, blk0, blk1, tile0, tile1, pad_[3];
 };
 
-// Counts of the device-side work lists (bsys: the large systems of the inner
-// list, whose scalars one CTA per system reduces).
+// A system in diagonal form (dia.cuh): at most kSysDiag diagonals, the entries
+// of each in ascending rows; constant: each diagonal holds one number.
+constexpr int kSysDiag = 8;
+struct alignas(16) SysDia {
+    int32_t off[kSysDiag];
+    double cval[kSysDiag];
+    int64_t base, ld;  // values that vary: entry (diagonal k, row i) at base + k ld + i
+    int32_t ndiag, constant;
+};
+
+// Counts of the device-side work lists.  The inner block list holds iblk
+// blocks of systems without a diagonal form, then those of systems with one
+// (all_blk together); the inner tile list the dtile tiles of the latter first.
+// bsys: the large systems without the form, whose alpha a CTA each reduces.
 struct ListHdr {
-    int32_t iblk, itile, isys, oblk, otile, osys, bsys, pad_;
+    int32_t iblk, itile, isys, oblk, otile, osys, bsys, dtile, all_blk, pad_[3];
 };
 
 // Control words of a step's device-side loop: the iterations done so far in
@@ -465,6 +477,203 @@ __global__ void __launch_bounds__(kWideThreads)
     }
 }
 
+// Inner iteration, step 1 for the systems in diagonal form: Ap = A p and p.Ap
+// per 256-row block, a row per thread -- the sums, and so the bits, of the
+// pipeline kernel's thread rows.  A CTA takes 1 / 2^split of a tile, two
+// blocks at a time; no column index is read and nothing staged: p comes
+// through L1 by the system's offsets, the values diagonal by diagonal, 32 rows
+// to a load (evict-first, so that the vectors stay in L2), or not at all in the
+// constant form.  The system (a large one) has its alpha reduced by the last of
+// its CTAs to finish, which saves bs_alpha's launch.
+//
+// 128^3, FP32, varying values: 19.7 us with the alpha, where the pipeline
+// kernel took 30.1 us and bs_alpha 5.1.  A CTA's first loads depend on one another (tile,
+// system, masks and p), so a few blocks to a CTA: 54 us with one, 33 with two,
+// 25 with four, 23 with eight (in a loop of its own).  One persistent grid
+// over all tiles needs 95 registers for the system at hand: 31 us.  Forming
+// p = z + beta p here, as the plain CG's graph path does, takes bs_pupdate's 4
+// us off and puts 6 on (25.4 us; 46.2 against 42.0 us per iteration).
+constexpr int kUnitBlocks = 8;  // row blocks of a CTA, at most (split >= 1)
+
+template <typename V, typename T, int KC, bool CONST>
+__device__ __forceinline__ void dia_unit(const int32_t (&offs)[kSysDiag],
+                                         const double* __restrict__ cval, int nd, const V* vp,
+                                         int64_t ld, int32_t row_begin, int32_t row_end,
+                                         uint32_t m0, uint32_t m1,
+                                         const uint8_t* __restrict__ mask,
+                                         const T* __restrict__ p, T* __restrict__ Ap,
+                                         T (*dots)[kThreads]) {
+    constexpr int R = sizeof(T) == 8 ? 1 : 2;  // rows of a thread at a time
+    const int t = threadIdx.x;
+    const uint32_t full_mask = (1u << nd) - 1u;
+    int32_t off[KC];
+    T cv[KC];
+#pragma unroll
+    for (int k = 0; k < KC; ++k) {
+        off[k] = offs[k];
+        cv[k] = CONST ? static_cast<T>(__ldg(cval + k)) : T(0);
+    }
+    uint32_t m[R];
+    m[0] = m0;
+    if constexpr (R > 1) m[R - 1] = m1;
+    int b = 0;
+    for (int32_t row0 = row_begin + t; row0 - t < row_end; row0 += R * kThreads, b += R) {
+        T x[R][KC], v[R][KC], pr[R];
+        bool full[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int32_t row = row0 + r * kThreads;
+            full[r] = KC == nd && __all_sync(0xffffffffu, m[r] == full_mask);
+            const T* pp = p + row;
+            if (full[r]) {
+#pragma unroll
+                for (int k = 0; k < KC; ++k) {
+                    x[r][k] = __ldg(pp + off[k]);
+                    v[r][k] = CONST ? cv[k] : widen<V, T>(ld_value_cs(vp + k * ld + row));
+                }
+                pr[r] = __ldg(pp);
+            } else {
+#pragma unroll
+                for (int k = 0; k < KC; ++k) {
+                    x[r][k] = T(0);
+                    v[r][k] = cv[k];
+                    if (m[r] >> k & 1u) {
+                        x[r][k] = __ldg(pp + off[k]);
+                        if constexpr (!CONST)
+                            v[r][k] = widen<V, T>(ld_value_cs(vp + k * ld + row));
+                    }
+                }
+                pr[r] = row < row_end ? __ldg(pp) : T(0);
+            }
+        }
+        uint32_t mn[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int32_t nx = row0 + (R + r) * kThreads;
+            mn[r] = nx < row_end ? __ldg(mask + nx) : 0u;
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int32_t row = row0 + r * kThreads;
+            T acc = T(0);
+            if (full[r]) {
+#pragma unroll
+                for (int k = 0; k < KC; ++k) acc = add_rn(acc, mul_rn(v[r][k], x[r][k]));
+            } else {
+#pragma unroll
+                for (int k = 0; k < KC; ++k)
+                    if (m[r] >> k & 1u) acc = add_rn(acc, mul_rn(v[r][k], x[r][k]));
+            }
+            T dot = T(0);
+            if (row < row_end) {
+                Ap[row] = acc;
+                dot += pr[r] * acc;
+            }
+            if (b + r < kUnitBlocks) dots[b + r][t] = dot;
+            m[r] = mn[r];
+        }
+    }
+}
+
+template <typename V, typename T>
+__global__ void __launch_bounds__(kThreads)
+    bs_spmv_dia(const int4* __restrict__ tiles, const ListHdr* hdr, int split,
+                const SysDia* __restrict__ dia, const uint8_t* __restrict__ mask,
+                const V* __restrict__ dv, const T* __restrict__ p, T* __restrict__ Ap,
+                SysState* sys, const int2* sblk, double* part, int par) {
+    __shared__ T dots[kUnitBlocks][kThreads];
+    __shared__ double wsum[kUnitBlocks][kWarps];
+    __shared__ double2 red[kWarps + 1];
+    __shared__ bool last;
+    const int t = threadIdx.x;
+    const int32_t tile = int32_t(blockIdx.x) >> split;
+    const int32_t rows = kTileRows >> split;
+    const int4 tl = tiles[tile];
+    if (tile >= __ldcg(&hdr->dtile)) return;
+    const int32_t slot = tl.z;
+    const int32_t row_begin = tl.x + (int32_t(blockIdx.x) - (tile << split)) * rows;
+    const int32_t row_end = min(tl.y, row_begin + rows);
+    if (row_begin >= row_end) return;
+    // everything the tile leads to, in one round of loads
+    const uint32_t m0 = row_begin + t < row_end ? __ldg(mask + row_begin + t) : 0u;
+    const uint32_t m1 =
+        row_begin + t + kThreads < row_end ? __ldg(mask + row_begin + t + kThreads) : 0u;
+    const SysDia& sd = dia[slot];
+    const int4 o0 = __ldg(reinterpret_cast<const int4*>(sd.off));
+    const int4 o1 = __ldg(reinterpret_cast<const int4*>(sd.off) + 1);
+    const int32_t off[kSysDiag] = {o0.x, o0.y, o0.z, o0.w, o1.x, o1.y, o1.z, o1.w};
+    const int64_t base = __ldg(&sd.base), ld = __ldg(&sd.ld);
+    const int2 kind = __ldg(reinterpret_cast<const int2*>(&sd.ndiag));  // ndiag, constant
+    const int2 br = __ldg(sblk + slot);
+    const int32_t sys_row0 = sys[slot].row0;
+    if (sys_phase(sys, slot) != kSysInner) return;  // not written in this step
+    const int nd = kind.x;
+    auto unit = [&](auto kc, auto c) {
+        dia_unit<V, T, decltype(kc)::value, decltype(c)::value>(
+            off, sd.cval, nd, dv + (base - sys_row0), ld, row_begin, row_end, m0, m1, mask, p, Ap,
+            dots);
+    };
+    auto with = [&](auto c) {
+        if (nd <= 3) unit(std::integral_constant<int, 3>(), c);
+        else if (nd <= 5) unit(std::integral_constant<int, 5>(), c);
+        else if (nd <= 7) unit(std::integral_constant<int, 7>(), c);
+        else unit(std::integral_constant<int, 8>(), c);
+    };
+    if (kind.y) with(std::true_type());
+    else with(std::false_type());
+    const int nb = (row_end - row_begin + kThreads - 1) / kThreads;
+    {
+        // every block's warp sums at once, from the thread's own products
+        double v[kUnitBlocks];
+#pragma unroll
+        for (int b = 0; b < kUnitBlocks; ++b) v[b] = b < nb ? double(dots[b][t]) : 0.0;
+        multi_warp_sum<kUnitBlocks>(v);
+        if ((t & 3) == 0) wsum[(t & 31) >> 2][t >> 5] = v[0];
+    }
+    __syncthreads();
+    if (t < nb) {
+        double s = 0.0;
+#pragma unroll
+        for (int q = 0; q < kWarps; ++q) s += wsum[t][q];
+        part[br.x + (row_begin - sys_row0) / kThreads + t] = s;
+    }
+    __syncthreads();
+    if (t == 0) {  // acq_rel: this CTA's sums before its arrival, the others' before the last
+        unsigned int prev;
+        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;"
+                     : "=r"(prev)
+                     : "l"(&sys[slot].blk_arrivals), "r"(unsigned(nb))
+                     : "memory");
+        last = prev + unsigned(nb) == unsigned(br.y - br.x);
+    }
+    __syncthreads();
+    if (!last) return;
+    if (t == 0) sys[slot].blk_arrivals = 0u;
+    const double pAp = ordered_sum256<false>(part, br.x, br.y, red).x;
+    if (t == 0) sys[slot].alpha = pAp != 0.0 ? __ldcg(&sys[slot].rzp[par]) / pAp : 0.0;
+}
+
+// The masks of a system just admitted and (where they vary) its values by
+// diagonal, from its CSR arrays in the arena.
+template <typename V>
+__global__ void __launch_bounds__(kThreads)
+    bs_dia_fill(SysDia sd, int32_t row0, int32_t n, const int32_t* __restrict__ rp,
+                const int32_t* __restrict__ col, const V* __restrict__ vals,
+                uint8_t* __restrict__ mask, V* __restrict__ dv) {
+    for (int32_t i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) {
+        const int32_t row = row0 + i, z1 = rp[row + 1];
+        uint32_t m = 0;
+        int k = 0;  // columns ascend, so do their diagonals
+        for (int32_t z = rp[row]; z < z1; ++z) {
+            const int32_t d = col[z] - row;
+            while (k < kSysDiag - 1 && sd.off[k] != d) ++k;
+            m |= 1u << k;
+            if (!sd.constant) dv[sd.base + k * sd.ld + i] = vals[z];
+        }
+        mask[row] = static_cast<uint8_t>(m);
+    }
+}
+
 // ---- per-row vector steps over tiles {row0, row1, slot} ----------------------------
 //
 // A tile is up to kTileRows consecutive rows of one system; tiles start on
@@ -695,31 +904,21 @@ __device__ __forceinline__ void update_tile(int32_t i, const int4 tl, SysState* 
     if (threadIdx.x == 0) reinterpret_cast<double2*>(part_tile)[i] = t;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kThreads, 4)
-    bs_update(const int4* tiles, const int32_t* count, SysState* sys, const int2* sblk,
-              const int2* stile, const double* part_blk, const T* __restrict__ p,
-              const T* __restrict__ Ap, const T* __restrict__ dinv, T* __restrict__ r,
-              T* __restrict__ z, T* __restrict__ d, double* part_tile, int par, StepCtl* ctl) {
-    __shared__ double2 red[kWarps + 1];
-    __shared__ bool last;
-    const int32_t i = blockIdx.x;
-    if (i >= __ldcg(count)) return;
-    const int4 tl = tiles[i];
-    update_tile<T, false, false>(i, tl, sys, sblk, stile, part_blk, p, Ap, dinv, r, z, d,
-                                 part_tile, par, red);
-    if (!tl.w) return;  // a small system: its tile CTAs decide in step 3
-    // A large system's stopping test and beta, by the last of its tile CTAs
-    // to finish (its tile sums in ordered_sum256's order, as the persistent
-    // step forms them), so the iteration needs no kernel of its own for them.
-    SysState& S = sys[tl.z];
-    const int2 tr = __ldg(stile + tl.z);
+// A large system's stopping test and beta, by the last of its tile CTAs
+// to finish (its tile sums in ordered_sum256's order, as the persistent
+// step forms them), so the iteration needs no kernel of its own for them.
+// Every thread of a tile CTA calls it, after the tile's sums are written.
+__device__ __forceinline__ void large_system_test(int32_t slot, SysState* sys, const int2* stile,
+                                                  const double* part_tile, int par, StepCtl* ctl,
+                                                  double2* red, bool* last) {
+    SysState& S = sys[slot];
+    const int2 tr = __ldg(stile + slot);
     if (threadIdx.x == 0) {
         __threadfence();  // this CTA's tile sum (and iteration count) before its arrival
-        last = atomicAdd(&S.tile_arrivals, 1u) == unsigned(tr.y - tr.x - 1);
+        *last = atomicAdd(&S.tile_arrivals, 1u) == unsigned(tr.y - tr.x - 1);
     }
     __syncthreads();
-    if (!last) return;
+    if (!*last) return;
     __threadfence();
     if (threadIdx.x == 0) S.tile_arrivals = 0u;
     if (__ldcg(&S.phase) != kSysInner) return;  // uniform over the CTA
@@ -741,6 +940,22 @@ __global__ void __launch_bounds__(kThreads, 4)
             if (ctl) atomicAdd(&ctl->live, 1u);
         }
     }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kThreads, 4)
+    bs_update(const int4* tiles, const int32_t* count, SysState* sys, const int2* sblk,
+              const int2* stile, const double* part_blk, const T* __restrict__ p,
+              const T* __restrict__ Ap, const T* __restrict__ dinv, T* __restrict__ r,
+              T* __restrict__ z, T* __restrict__ d, double* part_tile, int par, StepCtl* ctl) {
+    __shared__ double2 red[kWarps + 1];
+    __shared__ bool last;
+    const int32_t i = blockIdx.x;
+    if (i >= __ldcg(count)) return;
+    const int4 tl = tiles[i];
+    update_tile<T, false, false>(i, tl, sys, sblk, stile, part_blk, p, Ap, dinv, r, z, d,
+                                 part_tile, par, red);
+    if (tl.w) large_system_test(tl.z, sys, stile, part_tile, par, ctl, red, &last);
 }
 
 // Inner iteration, step 3, for tile i: (r.z, r.r) of the system from its tile
@@ -1007,6 +1222,8 @@ struct HostSys {
     int32_t phase = kSysFree;
     std::vector<BlockDesc> blocks;  // arena-global
     std::vector<int4> tiles;
+    bool dia = false;  // in diagonal form
+    int64_t dv0 = 0, dv_alloc = 0;  // its range of the values by diagonal (0: none)
 };
 
 }  // namespace nm
@@ -1024,6 +1241,13 @@ struct nm_solver {
     std::vector<nm::HostSys> sys;
     // arena (device)
     int32_t* rp = nullptr;     // [cap_rows + 16]
+    uint8_t* mask = nullptr;   // [cap_rows + 16] diagonals of a row (systems in diagonal form)
+    nm::SysDia* dia = nullptr;  // [cap_sys]
+    // inner values by diagonal, allocated when the first system needs them (a
+    // system that finds no room there runs from its CSR arrays)
+    void* dv = nullptr;
+    bool dv_tried = false;
+    nm::RangeAlloc dvals;
     int32_t* col = nullptr;    // [cap_nnz + 16]
     double* v64 = nullptr;     // [cap_nnz + 16]
     void* vin = nullptr;       // inner values [cap_nnz + 16] (float / bf16 / unused for FP64)
@@ -1045,10 +1269,18 @@ struct nm_solver {
     int4* h_tile = nullptr;
     nm::SysRef* h_ref = nullptr;
     bool lists_dirty = true;
-    // CUDA graph of one chunk of inner iterations; valid while the lists (and
-    // so every kernel argument) are unchanged
-    cudaGraphExec_t chunk_exec = nullptr;
-    bool chunk_valid = false;
+    // CUDA graphs of a step's loop, one for each set of kernels it can hold
+    // (bs_spmv_inner, bs_spmv_dia, bs_alpha: an executable graph takes other
+    // grids and arguments in place, not other kernels), each valid while what
+    // it was built against is unchanged
+    struct StepGraph {
+        cudaGraphExec_t exec = nullptr;
+        bool valid = false;
+        int64_t gen = -1;  // lists_gen
+        int tiles = 0;     // tile grid
+        int dia = 0;       // grid of bs_spmv_dia
+    };
+    StepGraph graphs[8];
     // nm_solver_take_batch: pinned landing of the solutions, slot lists
     double* take_stage = nullptr;
     size_t take_cap = 0;
@@ -1058,9 +1290,8 @@ struct nm_solver {
     int grid_spmv_inner = 0, grid_spmv_outer = 0, grid_vec = 0, grid_scalar = 0;
     int grid_persist = 0;     // co-resident grid of bs_persist (0: not available)
     int64_t lists_gen = 0;   // bumped when the work-list arrays are reallocated
-    int64_t graph_gen = -1;  // lists_gen the step graph was built against
-    int graph_tiles = 0;     // tile grid of the step graph
-    bool graph_big = false;  // the step graph includes bs_alpha
+    cudaStream_t side = nullptr;  // branch of the step graph's capture
+    cudaEvent_t fork = nullptr, join = nullptr;
     // pinned staging of admission uploads: a bump allocator, reset once the
     // stream has caught up (after each step's synchronisation)
     unsigned char* stage = nullptr;
@@ -1077,7 +1308,7 @@ struct nm_solver {
 };
 
 nm_solver::~nm_solver() {
-    cudaFree(rp); cudaFree(col); cudaFree(v64); cudaFree(vin);
+    cudaFree(rp); cudaFree(mask); cudaFree(dia); cudaFree(dv); cudaFree(col); cudaFree(v64); cudaFree(vin);
     cudaFree(b); cudaFree(x); cudaFree(r64);
     cudaFree(p); cudaFree(Ap); cudaFree(r); cudaFree(z); cudaFree(d); cudaFree(dinv);
     cudaFree(st); cudaFreeHost(h_st);
@@ -1087,7 +1318,8 @@ nm_solver::~nm_solver() {
     cudaFree(sblk); cudaFree(stile);
     cudaFreeHost(h_sblk); cudaFreeHost(h_stile);
     cudaFreeHost(h_blk); cudaFreeHost(h_tile); cudaFreeHost(h_ref); cudaFreeHost(stage);
-    if (chunk_exec) cudaGraphExecDestroy(chunk_exec);
+    for (StepGraph& g : graphs)
+        if (g.exec) cudaGraphExecDestroy(g.exec);
     cudaFree(ctl);
     cudaFreeHost(h_ctl);
     cudaFreeHost(take_stage);
@@ -1096,6 +1328,9 @@ nm_solver::~nm_solver() {
     if (up_ev) cudaEventDestroy(up_ev);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
+    if (fork) cudaEventDestroy(fork);
+    if (join) cudaEventDestroy(join);
+    if (side) cudaStreamDestroy(side);
     if (up) cudaStreamDestroy(up);
     if (stream) cudaStreamDestroy(stream);
 }
@@ -1157,31 +1392,47 @@ int upload_lists(nm_solver* S) {
     SysRef* ro = S->h_ref + S->cap_sys;
     SysRef* rb = S->h_ref + 2 * int64_t(S->cap_sys);
     int32_t cb_i = 0, ct_i = 0, cs_i = 0, cb_o = 0, ct_o = 0, cs_o = 0, cs_b = 0;
-    for (int32_t slot = 0; slot < S->cap_sys; ++slot) {
-        HostSys& h = S->sys[slot];
-        if (!h.used || (h.phase != kSysInner && h.phase != kSysOuter)) continue;
-        SysRef a{slot, cb_i, cb_i + int32_t(h.blocks.size()), ct_i,
-                 ct_i + int32_t(h.tiles.size()), {0, 0, 0}};
-        std::memcpy(bi + cb_i, h.blocks.data(), sizeof(BlockDesc) * h.blocks.size());
-        std::memcpy(ti + ct_i, h.tiles.data(), sizeof(int4) * h.tiles.size());
-        S->h_sblk[slot] = make_int2(a.blk0, a.blk1);
-        S->h_stile[slot] = make_int2(a.tile0, a.tile1);
-        cb_i = a.blk1;
-        ct_i = a.tile1;
-        ri[cs_i++] = a;
-        if (!h.tiles.empty() && h.tiles[0].w) rb[cs_b++] = a;
-        if (h.phase == kSysOuter) {
-            SysRef o{slot, cb_o, cb_o + int32_t(h.blocks.size()), ct_o,
-                     ct_o + int32_t(h.tiles.size()), {0, 0, 0}};
-            std::memcpy(bo + cb_o, h.blocks.data(), sizeof(BlockDesc) * h.blocks.size());
-            std::memcpy(to + ct_o, h.tiles.data(), sizeof(int4) * h.tiles.size());
-            cb_o = o.blk1;
-            ct_o = o.tile1;
-            ro[cs_o++] = o;
+    // Blocks: systems without a diagonal form first (bs_spmv_inner's part of
+    // the list); tiles: those with one first (bs_spmv_dia's).
+    int32_t cb_csr = 0, ct_dia = 0, ct_all = 0;
+    for (const HostSys& h : S->sys)
+        if (h.used && h.dia && (h.phase == kSysInner || h.phase == kSysOuter))
+            ct_dia += int32_t(h.tiles.size());
+    ct_i = ct_dia;
+    for (int pass = 0; pass < 2; ++pass) {
+        if (pass == 1) {
+            cb_csr = cb_i;
+            ct_all = ct_i;
+            ct_i = 0;
+        }
+        for (int32_t slot = 0; slot < S->cap_sys; ++slot) {
+            HostSys& h = S->sys[slot];
+            if (!h.used || (h.phase != kSysInner && h.phase != kSysOuter)) continue;
+            if (h.dia != (pass == 1)) continue;
+            SysRef a{slot, cb_i, cb_i + int32_t(h.blocks.size()), ct_i,
+                     ct_i + int32_t(h.tiles.size()), {0, 0, 0}};
+            std::memcpy(bi + cb_i, h.blocks.data(), sizeof(BlockDesc) * h.blocks.size());
+            std::memcpy(ti + ct_i, h.tiles.data(), sizeof(int4) * h.tiles.size());
+            S->h_sblk[slot] = make_int2(a.blk0, a.blk1);
+            S->h_stile[slot] = make_int2(a.tile0, a.tile1);
+            cb_i = a.blk1;
+            ct_i = a.tile1;
+            ri[cs_i++] = a;
+            if (!h.dia && !h.tiles.empty() && h.tiles[0].w) rb[cs_b++] = a;
+            if (h.phase == kSysOuter) {
+                SysRef o{slot, cb_o, cb_o + int32_t(h.blocks.size()), ct_o,
+                         ct_o + int32_t(h.tiles.size()), {0, 0, 0}};
+                std::memcpy(bo + cb_o, h.blocks.data(), sizeof(BlockDesc) * h.blocks.size());
+                std::memcpy(to + ct_o, h.tiles.data(), sizeof(int4) * h.tiles.size());
+                cb_o = o.blk1;
+                ct_o = o.tile1;
+                ro[cs_o++] = o;
+            }
         }
     }
     cudaStream_t s = S->stream;
-    *S->h_hdr = ListHdr{cb_i, ct_i, cs_i, cb_o, ct_o, cs_o, cs_b, 0};
+    ct_i = ct_all;
+    *S->h_hdr = ListHdr{cb_csr, ct_i, cs_i, cb_o, ct_o, cs_o, cs_b, ct_dia, cb_i, {0, 0, 0}};
     NM_CUDA_TRY(cudaMemcpyAsync(S->hdr, S->h_hdr, sizeof(ListHdr), cudaMemcpyHostToDevice, s));
     if (cb_i) NM_CUDA_TRY(cudaMemcpyAsync(S->iblk, bi, sizeof(BlockDesc) * cb_i, cudaMemcpyHostToDevice, s));
     if (cb_o) NM_CUDA_TRY(cudaMemcpyAsync(S->oblk, bo, sizeof(BlockDesc) * cb_o, cudaMemcpyHostToDevice, s));
@@ -1242,6 +1493,18 @@ int tile_bucket(int64_t tiles) {
     return int(std::min<int64_t>(b, INT32_MAX));
 }
 
+// bs_spmv_dia's CTAs per tile, as a power of two: enough of them for the GPU,
+// from two (2,048 rows each) to one per row block.
+int dia_split(int64_t tiles) {
+    int split = 1;
+    while (split < 4 && (int64_t(tile_bucket(tiles)) << split) < 512) ++split;
+    return split;
+}
+
+int dia_grid(int64_t tiles) {
+    return tiles > 0 ? tile_bucket(tiles) << dia_split(tiles) : 0;
+}
+
 // Grid of a persistent kernel over `count` items (at least one CTA).
 int fit_grid(int cap, int64_t count) {
     return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(cap, count)));
@@ -1261,6 +1524,8 @@ int launch_inner_body(nm_solver* S, cudaGraphConditionalHandle loop) {
     const int g_spmv = S->grid_spmv_inner;
     const int g_vec = tile_bucket(h.itile);
     const int g_big = h.bsys > 0 ? S->grid_scalar : 0;
+    const int split = dia_split(h.dtile);
+    const int g_dia = dia_grid(h.dtile);
     const CsrView<V> M = arena_view<V>(S, S->vin ? S->vin : S->v64, S->iblk, &H->iblk);
     constexpr size_t smem = spmv_smem_bytes<V, T, T, kSolverTile, kSolverStages>();
     T* p = static_cast<T*>(S->p);
@@ -1273,10 +1538,24 @@ int launch_inner_body(nm_solver* S, cudaGraphConditionalHandle loop) {
         const int par = it & 1;
         // the last iteration of the body counts the systems that go on
         StepCtl* ctl = it == kLoopUnroll - 1 ? S->ctl : nullptr;
-        bs_spmv_inner<V, T><<<g_spmv, kCtaThreads, smem, s>>>(M, p, Ap, S->st, S->part_blk,
-                                                              S->err);
+        // the two kinds of systems side by side
+        if (g_dia && h.iblk > 0) {
+            NM_CUDA_TRY(cudaEventRecord(S->fork, s));
+            NM_CUDA_TRY(cudaStreamWaitEvent(S->side, S->fork, 0));
+        }
+        if (h.iblk > 0)
+            bs_spmv_inner<V, T><<<g_spmv, kCtaThreads, smem, s>>>(M, p, Ap, S->st, S->part_blk,
+                                                                  S->err);
+        if (g_dia)
+            bs_spmv_dia<V, T><<<g_dia, kThreads, 0, h.iblk > 0 ? S->side : s>>>(
+                S->itile, H, split, S->dia, S->mask, static_cast<const V*>(S->dv), p, Ap, S->st,
+                S->sblk, S->part_blk, par);
         if (g_big) bs_alpha<<<g_big, kWideThreads, 0, s>>>(S->bsys, &H->bsys, S->st,
                                                            S->part_blk, par);
+        if (g_dia && h.iblk > 0) {
+            NM_CUDA_TRY(cudaEventRecord(S->join, S->side));
+            NM_CUDA_TRY(cudaStreamWaitEvent(s, S->join, 0));
+        }
         bs_update<T><<<g_vec, kThreads, 0, s>>>(S->itile, &H->itile, S->st, S->sblk, S->stile,
                                                 S->part_blk, p, Ap, dinv, r, z, d, S->part_tile,
                                                 par, ctl);
@@ -1324,6 +1603,8 @@ int prepare_solver_kernels(nm_solver* S) {
     NM_CUDA_TRY(cudaFuncGetAttributes(&fa, bs_pupdate<T>));
     NM_CUDA_TRY(cudaFuncGetAttributes(&fa, bs_pstart<T>));
     NM_CUDA_TRY(cudaFuncGetAttributes(&fa, bs_alpha));
+    NM_CUDA_TRY(cudaFuncGetAttributes(&fa, bs_spmv_dia<V, T>));
+    NM_CUDA_TRY(cudaFuncGetAttributes(&fa, bs_dia_fill<V>));
     NM_CUDA_TRY(cudaFuncGetAttributes(&fa, bs_control));
     NM_CUDA_TRY(cudaFuncGetAttributes(&fa, bs_free_slots));
     int st = prepare_kernel(reinterpret_cast<const void*>(bs_spmv_inner<V, T>), kCtaThreads,
@@ -1354,7 +1635,7 @@ int prepare_solver_kernels(nm_solver* S) {
 template <typename V, typename T>
 int launch_persist(nm_solver* S) {
     const ListHdr* H = S->hdr;
-    CsrView<V> M = arena_view<V>(S, S->vin ? S->vin : S->v64, S->iblk, &H->iblk);
+    CsrView<V> M = arena_view<V>(S, S->vin ? S->vin : S->v64, S->iblk, &H->all_blk);
     T* p = static_cast<T*>(S->p);
     T* Ap = static_cast<T*>(S->Ap);
     const T* dinv = static_cast<const T*>(S->dinv);
@@ -1437,6 +1718,10 @@ extern "C" int nm_solver_create(int64_t max_rows, int64_t max_nnz, int32_t max_s
     const size_t tb = inner_bytes(S->inner);
     NM_CUDA_TRY(cudaMalloc(&S->rp, sizeof(int32_t) * R));
     NM_CUDA_TRY(cudaMemset(S->rp, 0, sizeof(int32_t) * R));
+    NM_CUDA_TRY(cudaMalloc(&S->mask, R));
+    NM_CUDA_TRY(cudaMemset(S->mask, 0, R));
+    NM_CUDA_TRY(cudaMalloc(&S->dia, sizeof(SysDia) * size_t(max_systems)));
+    NM_CUDA_TRY(cudaMemset(S->dia, 0, sizeof(SysDia) * size_t(max_systems)));
     NM_CUDA_TRY(cudaMalloc(&S->col, sizeof(int32_t) * Z));
     NM_CUDA_TRY(cudaMemset(S->col, 0, sizeof(int32_t) * Z));
     NM_CUDA_TRY(cudaMalloc(&S->v64, sizeof(double) * Z));
@@ -1480,6 +1765,9 @@ extern "C" int nm_solver_create(int64_t max_rows, int64_t max_nnz, int32_t max_s
     NM_CUDA_TRY(cudaMallocHost(&S->stage, S->stage_cap));
     NM_CUDA_TRY(cudaStreamCreateWithFlags(&S->stream, cudaStreamNonBlocking));
     NM_CUDA_TRY(cudaStreamCreateWithFlags(&S->up, cudaStreamNonBlocking));
+    NM_CUDA_TRY(cudaStreamCreateWithFlags(&S->side, cudaStreamNonBlocking));
+    NM_CUDA_TRY(cudaEventCreateWithFlags(&S->fork, cudaEventDisableTiming));
+    NM_CUDA_TRY(cudaEventCreateWithFlags(&S->join, cudaEventDisableTiming));
     NM_CUDA_TRY(cudaEventCreateWithFlags(&S->up_ev, cudaEventDisableTiming));
     NM_CUDA_TRY(cudaEventCreate(&S->ev0));
     NM_CUDA_TRY(cudaEventCreate(&S->ev1));
@@ -1551,13 +1839,15 @@ struct AdmitJob {
     bool bad_rp = false;  // row_ptr decreases somewhere
     std::vector<BlockDesc> blocks;
     std::vector<int4> tiles;
+    bool dia = false;
 };
 
 size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 
 // Staging layout of a job: row_ptr, col_idx, FP64 values, inner values, b,
-// x0, inverse diagonal, SysState.
-void stage_sizes(const nm_solver* S, const AdmitJob& J, size_t sz[8]) {
+// x0, inverse diagonal, SysState, SysDia.
+constexpr int kStageParts = 9;
+void stage_sizes(const nm_solver* S, const AdmitJob& J, size_t sz[kStageParts]) {
     const size_t n = size_t(J.n), nz = size_t(J.row_ptr[J.n]);
     sz[0] = align256(sizeof(int32_t) * (n + 1));
     sz[1] = align256(sizeof(int32_t) * nz);
@@ -1567,10 +1857,11 @@ void stage_sizes(const nm_solver* S, const AdmitJob& J, size_t sz[8]) {
     sz[5] = align256(J.x0 ? sizeof(double) * n : 0);
     sz[6] = align256(inner_bytes(S->inner) * n);
     sz[7] = align256(sizeof(SysState));
+    sz[8] = align256(sizeof(SysDia));
 }
 
 size_t stage_total(const nm_solver* S, const AdmitJob& J) {
-    size_t sz[8];
+    size_t sz[kStageParts];
     stage_sizes(S, J, sz);
     size_t t = 0;
     for (size_t q : sz) t += q;
@@ -1625,10 +1916,110 @@ void job_release(nm_solver* S, AdmitJob& J) {
     J.slot = -1;
 }
 
+// A value as the inner precision holds it.
+double inner_value(int inner, double v) {
+    if (inner == NM_F64) return v;
+    if (inner == NM_F32) return static_cast<float>(v);
+    uint16_t h;
+    to_bf16(&v, 1, &h);
+    const uint32_t u = uint32_t(h) << 16;
+    float f;
+    std::memcpy(&f, &u, 4);
+    return f;
+}
+
+// The diagonals col - row of 64 rows spread over the matrix, ascending, each
+// with the value of one entry; false when they are too many, or a row too long
+// for whole 256-row blocks.
+bool look_for_diagonals(const int32_t* rp, const int32_t* ci, const double* val, int32_t n,
+                        SysDia* sd) {
+    constexpr int kLook = 64;
+    int nd = 0;
+    for (int q = 0; q < kLook; ++q) {
+        const int32_t r = static_cast<int32_t>(int64_t(n - 1) * q / (kLook - 1));
+        if (rp[r + 1] - rp[r] > kSysDiag) return false;
+        for (int32_t j = rp[r]; j < rp[r + 1]; ++j) {
+            const int64_t d = int64_t(ci[j]) - r;
+            if (ci[j] < 0 || ci[j] >= n) return false;
+            int k = 0;
+            while (k < nd && sd->off[k] < d) ++k;
+            if (k < nd && sd->off[k] == d) continue;
+            if (nd == kSysDiag) return false;
+            for (int e = nd; e > k; --e) {
+                sd->off[e] = sd->off[e - 1];
+                sd->cval[e] = sd->cval[e - 1];
+            }
+            sd->off[k] = static_cast<int32_t>(d);
+            sd->cval[k] = val[j];
+            ++nd;
+        }
+    }
+    sd->ndiag = nd;
+    return nd > 0;
+}
+
+// Whether the rows [i0, i1) ascend along sd's diagonals; *same: the entries of
+// each diagonal are one number there.
+bool along_diagonals(const int32_t* rp, const int32_t* ci, const double* val, int64_t i0,
+                     int64_t i1, const SysDia& sd, bool* same) {
+    int32_t off[kSysDiag + 1];
+    double cv[kSysDiag + 1] = {};
+    for (int k = 0; k <= kSysDiag; ++k) {
+        off[k] = k < sd.ndiag ? sd.off[k] : INT32_MAX;
+        if (k < sd.ndiag) cv[k] = sd.cval[k];
+    }
+    bool eq = true;
+    for (int64_t i = i0; i < i1; ++i) {
+        int k = 0;
+        const int32_t z1 = rp[i + 1];
+        for (int32_t j = rp[i]; j < z1; ++j, ++k) {
+            const int64_t d = int64_t(ci[j]) - i;
+            while (off[k] < d) ++k;
+            if (off[k] != d) return false;
+            eq &= val[j] == cv[k];
+        }
+    }
+    *same = eq;
+    return true;
+}
+
+// The x windows (see BlockDesc) of rows [b0, b1) of a system in diagonal form
+// at arena row r0: along each diagonal the columns those rows can have.
+void dia_windows(const SysDia& sd, int32_t b0, int32_t b1, int32_t r0, int32_t n,
+                 int32_t cap_rows, int4* xs, int4* xl) {
+    *xs = make_int4(-1, INT_MAX, INT_MAX, INT_MAX);
+    *xl = make_int4(0, 0, 0, 0);
+    int32_t st[kXSeg], en[kXSeg];
+    int nseg = 0;
+    for (int k = 0; k < sd.ndiag; ++k) {  // ascending
+        const int64_t lo = std::max<int64_t>(0, int64_t(b0) + sd.off[k]);
+        const int64_t hi = std::min<int64_t>(n, int64_t(b1) + sd.off[k]);
+        if (hi <= lo) continue;
+        const int32_t a = int32_t(r0 + lo) & ~3, e = int32_t(r0 + hi + 3) & ~3;
+        if (nseg > 0 && a <= en[nseg - 1] + kXGap) {
+            en[nseg - 1] = std::max(en[nseg - 1], e);
+            continue;
+        }
+        if (nseg == kXSeg) return;  // too many windows: gather from global
+        st[nseg] = a;
+        en[nseg++] = e;
+    }
+    int64_t total = 0;
+    for (int k = 0; k < nseg; ++k) total += en[k] - st[k];
+    if (nseg == 0 || total > xwin_capacity(kSolverTile) || en[nseg - 1] > (cap_rows & ~3)) return;
+    int32_t sv[kXSeg] = {INT_MAX, INT_MAX, INT_MAX, INT_MAX}, lv[kXSeg] = {0, 0, 0, 0};
+    for (int k = 0; k < nseg; ++k) {
+        sv[k] = st[k];
+        lv[k] = en[k] - st[k];
+    }
+    *xs = make_int4(sv[0], sv[1], sv[2], sv[3]);
+    *xl = make_int4(lv[0], lv[1], lv[2], lv[3]);
+}
+
 // Host preparation of one job into its staging; touches nothing shared, so
 // jobs run concurrently.  `inner_threads`: parallelise this job's rows.
 void job_prep(const nm_solver* S, AdmitJob& J, bool inner_threads) {
-    size_t sz[8];
+    size_t sz[kStageParts];
     stage_sizes(S, J, sz);
     unsigned char* q = J.stage;
     int32_t* grp = reinterpret_cast<int32_t*>(q); q += sz[0];
@@ -1638,7 +2029,8 @@ void job_prep(const nm_solver* S, AdmitJob& J, bool inner_threads) {
     double* bs = reinterpret_cast<double*>(q); q += sz[4];
     double* x0s = reinterpret_cast<double*>(q); q += sz[5];
     void* dinvs = q; q += sz[6];
-    SysState* ss = reinterpret_cast<SysState*>(q);
+    SysState* ss = reinterpret_cast<SysState*>(q); q += sz[7];
+    SysDia* sd = reinterpret_cast<SysDia*>(q);
     const int32_t n = J.n;
     const int32_t* rp = J.row_ptr;
     const int32_t* ci = J.col_idx;
@@ -1653,6 +2045,14 @@ void job_prep(const nm_solver* S, AdmitJob& J, bool inner_threads) {
             return;
         }
     std::mutex mu;
+    // The diagonals that a look at some rows shows; the system is in diagonal
+    // form when every row's columns ascend along them.
+    std::memset(sd, 0, sizeof(SysDia));
+    // (only where kernels are long: under a few hundred row blocks the pipeline
+    // kernel and alphas reduced by every tile CTA have less latency: 50^3 14.5
+    // us per iteration against 19)
+    const bool maybe_dia = n > kLargeBlocks * kThreads && look_for_diagonals(rp, ci, val, n, sd);
+    bool is_dia = maybe_dia, is_const = maybe_dia;
     auto rows = [&](int64_t i0, int64_t i1) {
         int badc = -1;
         for (int64_t i = i0; i < i1; ++i) {
@@ -1670,6 +2070,8 @@ void job_prep(const nm_solver* S, AdmitJob& J, bool inner_threads) {
             bs[i] = J.b[i];
             if (J.x0) x0s[i] = J.x0[i];
         }
+        bool on = maybe_dia, same = maybe_dia;
+        if (on) on = along_diagonals(rp, ci, val, i0, i1, *sd, &same);
         if (i1 > i0) {
             const size_t z0c = size_t(rp[i0]), nzc = size_t(rp[i1] - rp[i0]);
             std::memcpy(v64s + z0c, val + z0c, sizeof(double) * nzc);
@@ -1678,11 +2080,17 @@ void job_prep(const nm_solver* S, AdmitJob& J, bool inner_threads) {
         }
         std::lock_guard<std::mutex> g(mu);
         if (badc >= 0 && J.bad_col < 0) J.bad_col = badc;
+        is_dia = is_dia && on;
+        is_const = is_const && same;
     };
     if (inner_threads) parallel_for(n, 65536, rows);
     else rows(0, n);
     grp[n] = z0 + rp[n];
     if (J.bad_col >= 0) return;
+    J.dia = is_dia;
+    sd->constant = is_const ? 1 : 0;
+    for (int k = 0; k < sd->ndiag; ++k)  // as the inner iterations hold them
+        sd->cval[k] = inner_value(inner, sd->cval[k]);
     // |b|^2 in row order (the same bits however the rows were prepared)
     double bb = 0.0;
     for (int32_t i = 0; i < n; ++i) bb += J.b[i] * J.b[i];
@@ -1703,7 +2111,9 @@ void job_prep(const nm_solver* S, AdmitJob& J, bool inner_threads) {
                 nlong += (rp[rr + 1] - rp[rr]) > kDefaultShortMax;
             dsc.rz = make_int4(r0 + blk[k], r0 + blk[k + 1], z0 + lz0, z0 + lz1);
             dsc.aux = make_int4(nlong, slot, 0, 0);
-            if (lz1 - lz0 > kSolverTile) {
+            if (J.dia) {
+                dia_windows(*sd, blk[k], blk[k + 1], r0, n, cap_rows, &dsc.xs, &dsc.xl);
+            } else if (lz1 - lz0 > kSolverTile) {
                 dsc.xs = make_int4(-1, INT_MAX, INT_MAX, INT_MAX);
                 dsc.xl = make_int4(0, 0, 0, 0);
             } else {
@@ -1732,13 +2142,37 @@ void job_prep(const nm_solver* S, AdmitJob& J, bool inner_threads) {
     ss->phase = kSysOuter;
 }
 
+// Room for `count` values by diagonal (their start; -1: none left).
+int64_t dia_value_room(nm_solver* S, int64_t count) {
+    if (!S->dv_tried) {
+        S->dv_tried = true;
+        const int64_t cap = S->cap_nnz + S->cap_nnz / 8 + 64;
+        if (cudaMalloc(&S->dv, inner_val_bytes(S->inner) * size_t(cap)) == cudaSuccess) {
+            S->dvals.init(cap);
+            for (auto& g : S->graphs) g.valid = false;  // they hold the pointer
+        } else {
+            cudaGetLastError();
+            S->dv = nullptr;
+        }
+    }
+    return S->dv ? S->dvals.alloc(count) : -1;
+}
+
+template <typename V>
+void launch_dia_fill(nm_solver* S, const SysDia& sd, int64_t r0, int32_t n) {
+    const int grid = int(std::min<int64_t>((int64_t(n) + kThreads - 1) / kThreads, 4096));
+    bs_dia_fill<V><<<grid, kThreads, 0, S->up>>>(sd, int32_t(r0), n, S->rp, S->col,
+                                                 static_cast<const V*>(S->vin ? S->vin : S->v64),
+                                                 S->mask, static_cast<V*>(S->dv));
+}
+
 // Asynchronous uploads of a prepared job and its host record.
 int job_commit(nm_solver* S, AdmitJob& J) {
-    size_t sz[8];
+    size_t sz[kStageParts];
     stage_sizes(S, J, sz);
     unsigned char* q = J.stage;
-    unsigned char* ptr[8];
-    for (int k = 0; k < 8; ++k) {
+    unsigned char* ptr[kStageParts];
+    for (int k = 0; k < kStageParts; ++k) {
         ptr[k] = q;
         q += sz[k];
     }
@@ -1763,6 +2197,27 @@ int job_commit(nm_solver* S, AdmitJob& J) {
     NM_CUDA_TRY(cudaMemsetAsync(static_cast<unsigned char*>(S->d) + tb * size_t(r0), 0, tb * n, s));
     NM_CUDA_TRY(cudaMemcpyAsync(static_cast<unsigned char*>(S->dinv) + tb * size_t(r0), ptr[6], tb * n,
                                 cudaMemcpyHostToDevice, s));
+    SysDia* sd = reinterpret_cast<SysDia*>(ptr[8]);
+    int64_t dv0 = 0, dv_alloc = 0;
+    if (J.dia && !sd->constant) {
+        sd->ld = J.nrows_alloc;
+        dv0 = dia_value_room(S, sd->ndiag * sd->ld);
+        if (dv0 >= 0) {
+            sd->base = dv0;
+            dv_alloc = sd->ndiag * sd->ld;
+        } else {
+            J.dia = false;
+        }
+    }
+    if (J.dia) {
+        NM_CUDA_TRY(cudaMemcpyAsync(S->dia + J.slot, sd, sizeof(SysDia), cudaMemcpyHostToDevice, s));
+        switch (S->inner) {
+            case NM_F64: launch_dia_fill<double>(S, *sd, r0, J.n); break;
+            case NM_F32: launch_dia_fill<float>(S, *sd, r0, J.n); break;
+            default: launch_dia_fill<__nv_bfloat16>(S, *sd, r0, J.n); break;
+        }
+        NM_CHECK_LAUNCH();
+    }
     const SysState* ss = reinterpret_cast<const SysState*>(ptr[7]);
     S->h_st[J.slot] = *ss;
     NM_CUDA_TRY(cudaMemcpyAsync(S->st + J.slot, ss, sizeof(SysState), cudaMemcpyHostToDevice, s));
@@ -1776,6 +2231,9 @@ int job_commit(nm_solver* S, AdmitJob& J) {
     h.phase = kSysOuter;
     h.blocks = std::move(J.blocks);
     h.tiles = std::move(J.tiles);
+    h.dia = J.dia;
+    h.dv0 = dv0;
+    h.dv_alloc = dv_alloc;
     h.init = *ss;
     S->lists_dirty = true;
     return NM_OK;
@@ -1943,8 +2401,10 @@ extern "C" int nm_solver_step_begin(nm_solver* S, int32_t iters) {
     } else if (iters > 0) {
         const bool big = S->h_hdr->bsys > 0;
         const int tiles = tile_bucket(S->h_hdr->itile);
-        if (!S->chunk_valid || S->graph_big != big || S->graph_tiles != tiles ||
-            S->graph_gen != S->lists_gen) {
+        const bool csr = S->h_hdr->iblk > 0;
+        const int dia = dia_grid(S->h_hdr->dtile);
+        auto& G = S->graphs[(csr ? 1 : 0) + (dia ? 2 : 0) + (big ? 4 : 0)];
+        if (!G.valid || G.tiles != tiles || G.dia != dia || G.gen != S->lists_gen) {
             S->ctr.graph_captures += 1;
             // The step graph: a WHILE node whose body is one iteration of every
             // live system, ended on the device by bs_control.  Rebuilt when the
@@ -1986,16 +2446,16 @@ extern "C" int nm_solver_step_begin(nm_solver* S, int32_t iters) {
                 return fail(NM_ERR_CUDA, "solver step capture failed: %s", cudaGetErrorString(ec));
             }
             bool updated = false;
-            if (S->chunk_exec) {
+            if (G.exec) {
                 cudaGraphExecUpdateResultInfo info;
-                updated = cudaGraphExecUpdate(S->chunk_exec, g, &info) == cudaSuccess;
+                updated = cudaGraphExecUpdate(G.exec, g, &info) == cudaSuccess;
                 cudaGetLastError();  // an update refusal is not an error
             }
             if (!updated) {
                 S->ctr.graph_instantiations += 1;
-                if (S->chunk_exec) cudaGraphExecDestroy(S->chunk_exec);
-                S->chunk_exec = nullptr;
-                const cudaError_t ei = cudaGraphInstantiate(&S->chunk_exec, g, 0);
+                if (G.exec) cudaGraphExecDestroy(G.exec);
+                G.exec = nullptr;
+                const cudaError_t ei = cudaGraphInstantiate(&G.exec, g, 0);
                 if (ei != cudaSuccess) {
                     cudaGraphDestroy(g);
                     return fail(NM_ERR_CUDA, "solver chunk instantiate failed: %s",
@@ -2003,17 +2463,17 @@ extern "C" int nm_solver_step_begin(nm_solver* S, int32_t iters) {
                 }
             }
             cudaGraphDestroy(g);
-            S->chunk_valid = true;
-            S->graph_big = big;
-            S->graph_tiles = tiles;
-            S->graph_gen = S->lists_gen;
+            G.valid = true;
+            G.tiles = tiles;
+            G.dia = dia;
+            G.gen = S->lists_gen;
         }
         lap(S->ctr.s_capture);
         *S->h_ctl = StepCtl{};
         S->h_ctl->cap = unsigned(iters);
         NM_CUDA_TRY(cudaMemcpyAsync(S->ctl, S->h_ctl, sizeof(StepCtl), cudaMemcpyHostToDevice,
                                     S->stream));
-        NM_CUDA_TRY(cudaGraphLaunch(S->chunk_exec, S->stream));
+        NM_CUDA_TRY(cudaGraphLaunch(G.exec, S->stream));
         S->step_loops = true;
     }
     NM_CUDA_TRY(cudaEventRecord(S->ev1, S->stream));
@@ -2121,6 +2581,7 @@ extern "C" int nm_solver_take(nm_solver* S, int32_t slot, double* x_host) {
     NM_CUDA_TRY(cudaStreamSynchronize(S->stream));
     S->rows.release(h.row0, h.nrows_alloc);
     S->nnz.release(h.z0, h.nnz_alloc);
+    if (h.dv_alloc) S->dvals.release(h.dv0, h.dv_alloc);
     const bool was_active = h.phase == kSysInner || h.phase == kSysOuter;
     h = HostSys{};
     S->h_st[slot].phase = kSysFree;
@@ -2238,6 +2699,7 @@ extern "C" int nm_solver_take_batch(nm_solver* S, int32_t count, const int32_t* 
         off += size_t(h.n);
         S->rows.release(h.row0, h.nrows_alloc);
         S->nnz.release(h.z0, h.nnz_alloc);
+        if (h.dv_alloc) S->dvals.release(h.dv0, h.dv_alloc);
         if (h.phase == kSysInner || h.phase == kSysOuter) S->lists_dirty = true;
         h = HostSys{};
         S->h_st[slots[k]].phase = kSysFree;
