@@ -96,6 +96,9 @@ int nm_finalize(void);
  * returns NM_ERR_RUNTIME if any kernel gave up since the last call. */
 int nm_check_device_errors(void);
 
+/* Waits until the work queued on `stream` (a cudaStream_t) is done. */
+int nm_stream_wait(void* stream);
+
 /* Failure-detection hook for tests (no counterpart in the reference, whose
  * kernels have no bounded waits).  Runs the library's own bounded wait
  * routine in a kernel where the wait cannot complete -- kind 0: an mbarrier

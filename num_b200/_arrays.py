@@ -52,7 +52,7 @@ def device_array(a, dtype: str, name: str, ndim: int = 1):
         else:
             raise TypeError(f"{name}: expected a CUDA array (torch.Tensor, DLPack or "
                             f"__cuda_array_interface__), got {type(a).__name__}")
-    if t.device.type != "cuda":
+    if not t.is_cuda:
         raise TypeError(f"{name}: expected a CUDA array, got device {t.device}")
     if t.dtype != _TORCH_DTYPES[dtype]:
         raise TypeError(f"{name}: expected dtype {dtype}, got {t.dtype}")
@@ -64,5 +64,6 @@ def device_array(a, dtype: str, name: str, ndim: int = 1):
 
 
 def stream_of(t) -> int:
-    """cudaStream_t (as int) of torch's current stream on t's device."""
-    return torch.cuda.current_stream(t.device).cuda_stream
+    """cudaStream_t (as int) of torch's current stream on t's device, without
+    the Stream object that torch.cuda.current_stream builds (2.3 us)."""
+    return torch._C._cuda_getCurrentRawStream(t.get_device())

