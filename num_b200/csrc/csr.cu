@@ -4,6 +4,7 @@
 // rows-per-team pick of the reference custom kernel (src/spmv_kernel.hpp:102-109)
 // with a per-row-block partition computed once at upload.
 #include <algorithm>
+#include <atomic>
 #include <climits>
 #include <cstring>
 #include <string>
@@ -41,11 +42,12 @@ int build_row_blocks(const int32_t* rp, int32_t nrows, int tile, int max_rows, i
     return static_cast<int>(blk.size()) - 1;
 }
 
-void block_xwindows(const int32_t* ci, int32_t z0, int32_t z1, int32_t ncols, int xw,
+bool block_xwindows(const int32_t* ci, int32_t z0, int32_t z1, int32_t ncols, int xw,
                     std::vector<int32_t>& c, int4* xs, int4* xl) {
     *xs = make_int4(-1, INT_MAX, INT_MAX, INT_MAX);
     *xl = make_int4(0, 0, 0, 0);
-    if (z1 <= z0) return;
+    if (z1 <= z0) return true;
+    bool shared = false;
     int32_t cmin = ci[z0], cmax = ci[z0];
     for (int32_t j = z0 + 1; j < z1; ++j) {
         cmin = std::min(cmin, ci[j]);
@@ -54,15 +56,21 @@ void block_xwindows(const int32_t* ci, int32_t z0, int32_t z1, int32_t ncols, in
     const int64_t span = int64_t(cmax) - cmin + 1;
     if (span <= 64 * int64_t(z1 - z0)) {
         // narrow range: mark the columns in a bitmap, read them back in order
-        std::vector<uint64_t> bits(size_t((span + 63) / 64), 0);
+        const int32_t c0 = cmin & ~3;
+        std::vector<uint64_t> bits(size_t((span + (cmin - c0) + 63) / 64), 0);
         for (int32_t j = z0; j < z1; ++j) {
-            const int64_t o = ci[j] - cmin;
+            const int64_t o = ci[j] - c0;
             bits[size_t(o >> 6)] |= uint64_t(1) << (o & 63);
         }
         c.clear();
-        for (size_t w = 0; w < bits.size(); ++w)
+        int64_t groups = 0;
+        for (size_t w = 0; w < bits.size(); ++w) {
+            const uint64_t pairs = bits[w] | bits[w] >> 1;
+            groups += __builtin_popcountll((pairs | pairs >> 2) & 0x1111111111111111u);
             for (uint64_t m = bits[w]; m; m &= m - 1)
-                c.push_back(cmin + int32_t(w * 64 + size_t(__builtin_ctzll(m))));
+                c.push_back(c0 + int32_t(w * 64 + size_t(__builtin_ctzll(m))));
+        }
+        shared = 2 * groups <= z1 - z0;
     } else {
         c.assign(ci + z0, ci + z1);
         std::sort(c.begin(), c.end());
@@ -75,7 +83,7 @@ void block_xwindows(const int32_t* ci, int32_t z0, int32_t z1, int32_t ncols, in
         if (a <= ce + kXGap) {
             ce = std::max(ce, e);
         } else {
-            if (nseg == kXSeg) return;  // too many windows: gather from global
+            if (nseg == kXSeg) return shared;  // too many windows: gather from global
             st[nseg] = cs;
             en[nseg] = ce;
             ++nseg;
@@ -83,13 +91,13 @@ void block_xwindows(const int32_t* ci, int32_t z0, int32_t z1, int32_t ncols, in
             ce = e;
         }
     }
-    if (nseg == kXSeg) return;
+    if (nseg == kXSeg) return shared;
     st[nseg] = cs;
     en[nseg] = ce;
     ++nseg;
     int64_t total = 0;
     for (int k = 0; k < nseg; ++k) total += en[k] - st[k];
-    if (total > xw || en[nseg - 1] > (ncols & ~3)) return;  // too wide, or would read past x
+    if (total > xw || en[nseg - 1] > (ncols & ~3)) return shared;  // too wide, or would read past x
     int32_t sv[kXSeg] = {INT_MAX, INT_MAX, INT_MAX, INT_MAX}, lv[kXSeg] = {0, 0, 0, 0};
     for (int k = 0; k < nseg; ++k) {
         sv[k] = st[k];
@@ -97,6 +105,7 @@ void block_xwindows(const int32_t* ci, int32_t z0, int32_t z1, int32_t ncols, in
     }
     *xs = make_int4(sv[0], sv[1], sv[2], sv[3]);
     *xl = make_int4(lv[0], lv[1], lv[2], lv[3]);
+    return shared;
 }
 
 namespace {
@@ -193,8 +202,10 @@ int rebuild_blocks(nm_csr* A) {
     const int tile = A->tune.tile;
     const int short_max = A->tune.short_max;
     const int32_t nb = A->nblk, ncols = A->ncols;
+    std::atomic<int64_t> near{0};  // nonzeros of blocks that share lines of x
     auto fill = [&](int32_t b0, int32_t b1) {
         std::vector<int32_t> scratch;
+        int64_t mine = 0;
         for (int32_t b = b0; b < b1; ++b) {
             BlockDesc& d = desc[b];
             const int32_t z0 = rp[blk[b]], z1 = rp[blk[b + 1]];
@@ -206,9 +217,11 @@ int rebuild_blocks(nm_csr* A) {
                 d.xs = make_int4(-1, INT_MAX, INT_MAX, INT_MAX);
                 d.xl = make_int4(0, 0, 0, 0);
             } else {
-                block_xwindows(ci, z0, z1, ncols, xwin_capacity(tile), scratch, &d.xs, &d.xl);
+                if (block_xwindows(ci, z0, z1, ncols, xwin_capacity(tile), scratch, &d.xs, &d.xl))
+                    mine += z1 - z0;
             }
         }
+        near += mine;
     };
     const int nthr = static_cast<int>(std::min<int64_t>(
         std::max(1u, std::thread::hardware_concurrency()), std::max<int64_t>(1, nb / 256)));
@@ -235,6 +248,7 @@ int rebuild_blocks(nm_csr* A) {
                          A->tune.kernel == NM_KERNEL_SLICED ||
                          (A->tune.kernel == NM_KERNEL_AUTO && scattered);
     }
+    A->near_columns = 4 * near.load() >= 3 * int64_t(A->nnz);
     if (A->tune.kernel == NM_KERNEL_SLICED && !A->sell_tried) {
         const int st = build_sell(A);
         if (st != NM_OK) return st;

@@ -85,8 +85,9 @@ constexpr int kDefaultShortMax = 32;
 constexpr int kDefaultStages = 2;
 
 // x windows of the multi-row block with nonzeros [z0, z1) (see BlockDesc);
-// xw = largest total window length, ncols = length of x.
-void block_xwindows(const int32_t* col_idx, int32_t z0, int32_t z1, int32_t ncols, int xw,
+// xw = largest total window length, ncols = length of x.  True when the
+// nonzeros share lines of x (nm_csr::near_columns).
+bool block_xwindows(const int32_t* col_idx, int32_t z0, int32_t z1, int32_t ncols, int xw,
                     std::vector<int32_t>& scratch, int4* xs, int4* xl);
 
 // Row-block partition rule, shared by the device library and restated by the
@@ -132,6 +133,14 @@ struct nm_csr {
     // from tune.kernel (AUTO: most nonzeros in blocks without x windows and no
     // row longer than kWarpGatherMaxRow).
     bool warp_gather = false;
+    // At least 3/4 of the nonzeros are in blocks whose nonzeros fall on at
+    // most half as many aligned groups of 4 columns as there are nonzeros:
+    // the row-block kernel then reads x entries that have no window through
+    // L1, where only a line's first use costs an L2 access.  Banded systems
+    // with two random entries per row (48 M nonzeros): 162 -> 147 us;
+    // power-law rows took 149 us this way and 137 us past L1.  Its own kernel
+    // variant: with both reads in one kernel that case took 164 us.
+    bool near_columns = false;
     // The gather kernel's copy of the matrix (built the first time that kernel
     // is selected, kept until the handle is freed): rows sorted by length
     // (descending, stable) within windows of kSellWindow rows, cut into slices

@@ -8,14 +8,15 @@
 
 namespace nm {
 
-template <typename V, typename X, typename A, int TILE, int STAGES>
+// L1X: see nm_csr::near_columns.
+template <typename V, typename X, typename A, int TILE, int STAGES, bool L1X>
 __global__ void __launch_bounds__(kCtaThreads)
     spmv_kernel(const CsrView<V> M, const X* __restrict__ x, X* __restrict__ y,
                 unsigned int* err) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     auto& sm = *reinterpret_cast<SpmvSmem<V, X, A, TILE, STAGES>*>(smem_raw);
     StoreEpi<X, A> epi{y};
-    spmv_pipeline<V, X, A, TILE, STAGES>(M, x, sm, epi, err);
+    spmv_pipeline<V, X, A, TILE, STAGES, false, L1X>(M, x, sm, epi, err);
 }
 
 // ---------------------------------------------------------------------------
@@ -314,7 +315,8 @@ static int launch_tile(const nm_csr* Am, const X* x, X* y, cudaStream_t s, int32
     }
     M.stage_x = (reinterpret_cast<uintptr_t>(x) % 16) == 0;
     constexpr size_t smem = spmv_smem_bytes<V, X, A, TILE, STAGES>();
-    auto* fn = spmv_kernel<V, X, A, TILE, STAGES>;
+    auto* fn = Am->near_columns ? spmv_kernel<V, X, A, TILE, STAGES, true>
+                                : spmv_kernel<V, X, A, TILE, STAGES, false>;
     int occ = 0;
     int st = prepare_kernel(reinterpret_cast<const void*>(fn), kCtaThreads, smem, &occ);
     if (st != NM_OK) return st;

@@ -242,7 +242,7 @@ __device__ __forceinline__ A* prod_slots(SpmvStage<V, X, TILE>& st) {
     }
 }
 
-template <typename V, typename X, typename A, int TILE, int STAGES, bool XR, class Epi>
+template <bool L1X, typename V, typename X, typename A, int TILE, int STAGES, bool XR, class Epi>
 __device__ __forceinline__ void spmv_rows(const CsrView<V>& M, int s, bool ok, const BlockDesc& d,
                                           const X* __restrict__ x,
                                           SpmvSmem<V, X, A, TILE, STAGES, XR>& sm, Epi& epi,
@@ -290,12 +290,15 @@ __device__ __forceinline__ void spmv_rows(const CsrView<V>& M, int s, bool ok, c
             }
 #pragma unroll
             for (int g = 0; g < G; ++g)
-                // through L2 (ld.global.cg): scattered columns rarely hit L1,
+                // Through L2 (ld.global.cg): scattered columns rarely hit L1,
                 // and skipping it raises the gather rate (power-law rows:
-                // 299 -> 248 us per SpMV)
+                // 299 -> 248 us per SpMV).  With L1X through L1, where the
+                // rows of a block share lines of x (nm_csr::near_columns).
                 if (j0 + g * kConsumers < j1) {
                     if constexpr (XR)
                         xv[g] = static_cast<A>(fma(beta, __ldcg(x + c[g]), __ldcg(xr + c[g])));
+                    else if constexpr (L1X)
+                        xv[g] = static_cast<A>(__ldg(x + c[g]));
                     else
                         xv[g] = static_cast<A>(__ldcg(x + c[g]));
                 }
@@ -380,9 +383,10 @@ __device__ __forceinline__ void spmv_rows(const CsrView<V>& M, int s, bool ok, c
 // up (the error word is set; partial results must not be used).  On return
 // no TMA copy into this CTA's shared memory is pending.
 // With XR the vector multiplied is x' = fma(beta, x, xr), formed from staged
-// windows of both (or gathered pairs) as it is read.
-template <typename V, typename X, typename A, int TILE, int STAGES, bool XR = false, class Epi,
-          class Gate = AllBlocks>
+// windows of both (or gathered pairs) as it is read.  With L1X x entries
+// without a window are read through L1 (x must not change within the kernel).
+template <typename V, typename X, typename A, int TILE, int STAGES, bool XR = false,
+          bool L1X = false, class Epi, class Gate = AllBlocks>
 __device__ __forceinline__ bool spmv_pipeline(CsrView<V> M, const X* __restrict__ x,
                                               SpmvSmem<V, X, A, TILE, STAGES, XR>& sm, Epi& epi,
                                               unsigned int* err, const Gate& gate = Gate(),
@@ -488,7 +492,7 @@ __device__ __forceinline__ bool spmv_pipeline(CsrView<V> M, const X* __restrict_
             spmv_long_row<V, X, A, TILE, STAGES, XR>(M, active, d.rz.x, d.rz.z, d.rz.w, x, sm,
                                                      epi, xr, beta);
         else
-            spmv_rows<V, X, A, TILE, STAGES, XR>(M, s, active, d, x, sm, epi, xr, beta);
+            spmv_rows<L1X, V, X, A, TILE, STAGES, XR>(M, s, active, d, x, sm, epi, xr, beta);
         if constexpr (Epi::kBlockSums) {
             const double v = warp_sum(epi.take());
             if (lane == 0) sm.blk_red[s][warp] = v;  // published by the arrival below
