@@ -23,6 +23,12 @@
 //    sets of lines in turn, since a CTA may publish the next sums before a
 //    slower one has read these).  These two exchanges are all the
 //    synchronisation of an iteration; r travels under the second one.
+//  * Beyond kDiaCgTileSums tiles r travels as plain doubles instead, read two
+//    to a load behind a flag per CTA: the words' bytes and the instructions
+//    for them were what an iteration took there.  A CTA raises its flag (after
+//    a fence) and waits for those of the CTAs that hold its reach while the
+//    second sums travel.  Per iteration, with words -> with flags: 100^3
+//    19.5 -> 15.1 us, 90^3 17.6 -> 12.6, 80^3 11.5 -> 9.6, 1000^2 12.7 -> 10.7.
 //  * A line has one writer and is polled at one word: with the words of
 //    several CTAs in a line, or all of them polled, the polls held up the
 //    stores and each other (22,500 rows: 17,000 cycles for the two exchanges
@@ -49,6 +55,7 @@ constexpr int kDiaCgMaxDiag = 8;
 constexpr int64_t kDiaCgMinRows = 32768;
 constexpr size_t kDiaCgMaxSmem = 208 * 1024;
 constexpr int kDiaCgMaxGrid = 160;
+constexpr int kDiaCgSets = 3;  // sets of lines: two of sums in turn, one of flags
 constexpr int kDiaCgLine = 8;  // words of a CTA's line: its tiles, at most 8
 
 struct DiaCgArgs {
@@ -57,8 +64,8 @@ struct DiaCgArgs {
     CgState* st;
     const double* P0;  // p_0 = r_0 (the initial kernel)
     const double* R0;
-    ulonglong2* rword;  // per row: {r, iteration}
-    ulonglong2* lines;  // 2 x grid lines of {sum, exchange}
+    ulonglong2* rword;  // per row: {r, iteration}; without tile sums r alone, in 8 bytes
+    ulonglong2* lines;  // 2 x grid lines of {sum, exchange}, grid lines of {0, iteration}
     unsigned int* err;
     int32_t ntile, tiles_per_cta;
     int32_t early_r;  // shared memory has room for the r of other CTAs' rows
@@ -106,6 +113,7 @@ __host__ __device__ inline void dia_reach(const int32_t* off, int nd, int32_t n,
             out->nseg = s + 1;
             out->row[s] = a;
             out->len[s] = b - a;
+            total += (total ^ a) & 1;  // even rows at even slots
             out->base[s] = total;
             total += b - a;
         }
@@ -292,6 +300,10 @@ __global__ void __launch_bounds__(kDiaCgThreads, 1) cg_dia_kernel(const DiaCgArg
     extern __shared__ __align__(16) double pe[];  // the direction on DiaReach's rows
     __shared__ DiaExchange X;
     __shared__ DiaReach reach;
+    __shared__ int32_t near[2 * kDiaCgMaxDiag];
+    // the reach without the own rows: {first row, end row, slot - row, 0}
+    __shared__ int4 pieces[kDiaCgMaxDiag + 2];
+    __shared__ int32_t npiece, split;
     const int t = threadIdx.x;
     CgState* st = a.st;
     if (__ldcg(&st->done)) return;  // the initial kernel decided already
@@ -305,7 +317,32 @@ __global__ void __launch_bounds__(kDiaCgThreads, 1) cg_dia_kernel(const DiaCgArg
     const int32_t max_iter = __ldcg(&st->max_iter), guard = __ldcg(&st->guard);
     double rr = __ldcg(&st->rr);
     int32_t iter = __ldcg(&st->iter);
-    if (t == 0) dia_reach(a.D.off, a.ndiag, n, row0, row1, &reach);
+    if (t == 0) {
+        dia_reach(a.D.off, a.ndiag, n, row0, row1, &reach);
+        int np = 0;
+        for (int s = 0; s < reach.nseg; ++s) {
+            const int32_t first = reach.row[s], end = first + reach.len[s];
+            const int32_t shift = reach.base[s] - first;
+            const int32_t lo = min(end, row0), hi = max(first, row1);
+            if (first < lo) pieces[np++] = make_int4(first, lo, shift, 0);
+            if (hi < end) pieces[np++] = make_int4(hi, end, shift, 0);
+        }
+        npiece = np;
+        // the split nearest to half of the rows; none where one piece holds
+        // three quarters of them
+        int total = 0, best = 0, most = 0;
+        for (int s = 0; s < np; ++s) total += pieces[s].y - pieces[s].x;
+        most = total - total / 4;
+        for (int s = 1, before = 0; s < np; ++s) {
+            before += pieces[s - 1].y - pieces[s - 1].x;
+            const int larger = max(before, total - before);
+            if (larger < most) {
+                most = larger;
+                best = s;
+            }
+        }
+        split = best;
+    }
     __syncthreads();
     const int32_t own = reach.own;
 
@@ -341,6 +378,20 @@ __global__ void __launch_bounds__(kDiaCgThreads, 1) cg_dia_kernel(const DiaCgArg
             pe[reach.base[s] + e] = __ldcg(a.P0 + reach.row[s] + e);
     __syncthreads();
 
+    double* rplain = reinterpret_cast<double*>(a.rword);
+    ulonglong2* flags = a.lines + size_t(2) * gridDim.x * kDiaCgLine;
+    if (!TILES && t < 2 * kDiaCgMaxDiag) {  // the CTAs of each diagonal's first and last row
+        const int d = t >> 1;
+        int c = -1;
+        if (d < a.ndiag) {
+            const int64_t f = int64_t(row0) + a.D.off[d], l = int64_t(row1) - 1 + a.D.off[d];
+            if (l >= 0 && f < n) {
+                const int64_t row = t & 1 ? (l < n ? l : n - 1) : (f > 0 ? f : 0);
+                c = static_cast<int>(row / (int64_t(a.tiles_per_cta) * kThreads));
+            }
+        }
+        near[t] = c == int(blockIdx.x) ? -1 : c;
+    }
     uint64_t phase = 0;
     double beta = 0.0;
     bool failed = false;
@@ -438,7 +489,10 @@ __global__ void __launch_bounds__(kDiaCgThreads, 1) cg_dia_kernel(const DiaCgArg
                 if (q >= Q) continue;
                 if (have >> q & 1u) {
                     r[q] = fma(-alpha, ap[q], r[q]);  // r = -alpha*Ap + r
-                    if (shown >> q & 1u) st_word(a.rword + (row0 + q * NT + t), r[q], k);
+                    if (shown >> q & 1u) {
+                        if constexpr (TILES) st_word(a.rword + (row0 + q * NT + t), r[q], k);
+                        else __stcg(rplain + (row0 + q * NT + t), r[q]);
+                    }
                     x[q] = fma(alpha, pe[own + q * NT + t], x[q]);  // x = alpha*p + x
                     d[j] = fma(r[q], r[q], 0.0);
                 }
@@ -473,9 +527,59 @@ __global__ void __launch_bounds__(kDiaCgThreads, 1) cg_dia_kernel(const DiaCgArg
             }
         };
         double* hr = pe + reach.total;
+        // Without TILES: two rows to a load, from an even row on, eight loads
+        // in flight per thread; half of the threads take the pieces before
+        // `split`, the others the rest, so that two pieces are under way.
+        auto plain = [&] {
+            const bool both = split == 0, upper = !both && t >= NT / 2;
+            const int nt = both ? NT : NT / 2, tt = upper ? t - NT / 2 : t;
+            const int s1 = both || upper ? npiece : split;
+            for (int s = upper ? split : 0; s < s1; ++s) {
+                constexpr int N = 8;
+                const int4 pc = pieces[s];
+                const int32_t e1 = (pc.x & ~1) + 2 * tt;
+                double* const p2 = pe + pc.z;
+                for (int32_t e0 = e1; e0 < pc.y; e0 += 2 * nt * N) {
+                    double2 w[N];
+#pragma unroll
+                    for (int j = 0; j < N; ++j)
+                        if (e0 + 2 * nt * j < pc.y)
+                            w[j] = __ldcg(reinterpret_cast<const double2*>(rplain + e0 + 2 * nt * j));
+#pragma unroll
+                    for (int j = 0; j < N; ++j) {
+                        const int32_t e = e0 + 2 * nt * j;
+                        if (e >= pc.x && e + 1 < pc.y) {
+                            double2 v = *reinterpret_cast<double2*>(p2 + e);
+                            v.x = fma(beta, v.x, w[j].x);
+                            v.y = fma(beta, v.y, w[j].y);
+                            *reinterpret_cast<double2*>(p2 + e) = v;
+                        } else if (e >= pc.x && e < pc.y) {
+                            p2[e] = fma(beta, p2[e], w[j].x);
+                        } else if (e < pc.x && e + 1 < pc.y) {
+                            p2[e + 1] = fma(beta, p2[e + 1], w[j].y);
+                        }
+                    }
+                }
+            }
+        };
         auto early = [&](bool& ok) {
-            if (a.early_r) others(kThreads, std::integral_constant<int, 4>(), ok,
-                                   [&](int i, double rj) { hr[i] = rj; });
+            if constexpr (!TILES) {
+                // this CTA's flag, and those of the CTAs that hold its reach
+                if (t == kThreads) {
+                    __threadfence();
+                    st_word(flags + blockIdx.x * kDiaCgLine, 0.0, k);
+                } else if (t >= kThreads + 32 && t < kThreads + 32 + 2 * kDiaCgMaxDiag) {
+                    const int c = near[t - kThreads - 32];
+                    if (c >= 0) {
+                        const ulonglong2* f = flags + c * kDiaCgLine;
+                        wait_word(f, ld_word(f), k, a.err, &ok);
+                        __threadfence();
+                    }
+                }
+            } else if (a.early_r) {
+                others(kThreads, std::integral_constant<int, 4>(), ok,
+                       [&](int i, double rj) { hr[i] = rj; });
+            }
         };
         if (!gather<TILES>(a, phase, X, early, [&](double rr_new, double* sc) {
                 const double b = rr_new / rr;
@@ -495,7 +599,10 @@ __global__ void __launch_bounds__(kDiaCgThreads, 1) cg_dia_kernel(const DiaCgArg
         for (int q = 0; q < Q; ++q)
             if (have >> q & 1u)
                 pe[own + q * NT + t] = fma(beta, pe[own + q * NT + t], r[q]);
-        if (a.early_r) {
+        if constexpr (!TILES) {
+            plain();
+            __syncthreads();
+        } else if (a.early_r) {
             for (int s = 0; s < reach.nseg; ++s)
                 for (int e = t; e < reach.len[s]; e += NT) {
                     const int32_t row = reach.row[s] + e, i = reach.base[s] + e;
@@ -544,13 +651,15 @@ const void* dia_cg_k(bool tiles, int Q, bool constant) {
     }
     if (Q == 4) return reinterpret_cast<const void*>(cg_dia_kernel<4, KC, true, false>);
     if (Q == 8) return reinterpret_cast<const void*>(cg_dia_kernel<8, KC, true, false>);
+    if (Q == 11) return reinterpret_cast<const void*>(cg_dia_kernel<11, KC, true, false>);
     return reinterpret_cast<const void*>(cg_dia_kernel<14, KC, true, false>);
 }
 
-// Rows per thread of the kernel that takes `Q` (0: none does).
+// Rows per thread of the kernel that takes `Q` (0: none does).  11: 90^3, of
+// 10 rows per thread, takes 12.6 us per iteration, with the kernel for 14 15.9.
 int q_class(bool tiles, int Q) {
     if (tiles) return Q <= 1 ? 1 : (Q <= 2 ? 2 : (Q <= 4 ? 4 : 0));
-    return Q <= 4 ? 4 : (Q <= 8 ? 8 : (Q <= 14 ? 14 : 0));
+    return Q <= 4 ? 4 : (Q <= 8 ? 8 : (Q <= 11 ? 11 : (Q <= 14 ? 14 : 0)));
 }
 
 const void* dia_cg_kernel_for(const nm_csr* A, const CgWorkspace* ws) {
@@ -563,7 +672,8 @@ const void* dia_cg_kernel_for(const nm_csr* A, const CgWorkspace* ws) {
 }
 
 size_t dia_cg_bytes(const CgWorkspace* ws) {
-    return sizeof(ulonglong2) * (size_t(2 * kDiaCgLine) * size_t(ws->dia_grid) + size_t(ws->n));
+    return sizeof(ulonglong2) *
+           (size_t(kDiaCgSets * kDiaCgLine) * size_t(ws->dia_grid) + size_t(ws->n));
 }
 
 }  // namespace
@@ -601,9 +711,9 @@ int plan_dia(const nm_csr* A, CgWorkspace* ws) {
     }
     ws->dia_smem = sizeof(double) * size_t(total);
     if (ws->dia_smem > kDiaCgMaxSmem || ws->dia_grid > kDiaCgMaxGrid) return NM_OK;
-    // Other CTAs' r under the second exchange where rows are few (500^2: 7.9
-    // against 8.4 us per iteration) and by half the threads; beyond, by all of
-    // them after it (80^3: 11.4 against 13.5 us).
+    // Other CTAs' words of r under the second exchange, by half the threads,
+    // where shared memory has room (500^2: 7.9 against 8.4 us per iteration
+    // after it).
     ws->dia_early = ws->dia_tiles && 2 * ws->dia_smem <= kDiaCgMaxSmem;
     if (ws->dia_early) ws->dia_smem *= 2;
     const void* fn = dia_cg_kernel_for(A, ws);
@@ -633,7 +743,7 @@ int launch_dia_cg(const nm_csr* A, CgWorkspace* ws, cudaStream_t s) {
     a.P0 = ws->p;
     a.R0 = ws->r;
     a.lines = static_cast<ulonglong2*>(ws->dia_mem);
-    a.rword = a.lines + size_t(2 * kDiaCgLine) * ws->dia_grid;
+    a.rword = a.lines + size_t(kDiaCgSets * kDiaCgLine) * ws->dia_grid;
     a.err = ws->err;
     a.ntile = A->nblk;
     a.tiles_per_cta = ws->dia_b;

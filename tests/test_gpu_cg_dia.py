@@ -51,10 +51,13 @@ def _solve(kspmv, nmlib, M, b, mode, **kw):
 
 
 # one and two tiles per CTA, a ragged last tile, 2 and 4 rows per thread, the
-# last size with tile sums and the first without, 8 and 14 rows per thread
+# last size with tile sums and the first without, 4, 8, 11 and 14 rows per
+# thread; even and odd distances between a CTA's rows and those it reads
 @pytest.mark.parametrize("case", ["lap2d_182", "lap2d_200", "lap2d_256", "lap2d_301",
                                   "lap2d_512", "lap2d_513", "lap3d_33", "lap3d_58", "lap3d_80",
-                                  "lap2d_1029", "tridiag_40001", "tridiag_400001", "eight_50001",
+                                  "lap2d_600", "lap2d_1029", "lap3d_65", "lap3d_89", "lap3d_90",
+                                  "lap3d_101", "tridiag_40001", "tridiag_262145",
+                                  "tridiag_400001", "eight_50001", "eight_300001",
                                   "varcoef_33", "varcoef_64"])
 def test_diagonal_solve(kspmv, nmlib, case):
     name, size = case.split("_")
