@@ -65,6 +65,7 @@ bool block_xwindows(const int32_t* ci, int32_t z0, int32_t z1, int32_t ncols, in
         c.clear();
         int64_t groups = 0;
         for (size_t w = 0; w < bits.size(); ++w) {
+            if (!bits[w]) continue;
             const uint64_t pairs = bits[w] | bits[w] >> 1;
             groups += __builtin_popcountll((pairs | pairs >> 2) & 0x1111111111111111u);
             for (uint64_t m = bits[w]; m; m &= m - 1)
