@@ -5,7 +5,8 @@ Default workload (one step = one FP64 CSR SpMV, y = A x):
   3-D 7-point Laplacian on a 160^3 grid: n = 4,096,000, nnz = 28,518,400,
   int32 indices, FP64 values, x ~ U[-1, 1] (default_rng(1)).
   Algorithmic bytes per SpMV = 12 nnz + 4 (n + 1) + 8 n (x) + 8 n (y)
-  = 424.14 MB, larger than the 126 MB L2, so no flush is needed between steps.
+  = 424.14 MB by the CSR formula; the diagonal form moves 69.6 MB of them, less
+  than L2 holds, so L2 is flushed between steps.
   The default line also carries a `secondary` object: plain FP64 CG solves/s
   on the 256^2 Laplacian, the 160^3 matrix setup time (host build + upload
   against on-device assembly) and a served-CG sample (see serve_c5).
@@ -170,6 +171,23 @@ def block_diagonal(mats):
         z += A.nnz
     return Csr(np.concatenate(rps).astype(np.int32), np.concatenate(cis).astype(np.int32),
                np.concatenate(vals), r, r)
+
+
+def diagonal_form_bytes(A, precision):
+    """Bytes one SpMV moves when A is stored in diagonal form (at most 16
+    diagonals): masks, the values by diagonal unless each is one number, x and
+    y.  None for other matrices."""
+    row = np.repeat(np.arange(A.nrows, dtype=np.int64), np.diff(A.row_ptr))
+    d = A.col_idx - row
+    if len(np.unique(d[:4096])) > 16 or len(np.unique(d[-4096:])) > 16:
+        return None
+    off = np.flatnonzero(np.bincount(d + A.nrows))
+    if len(off) > 16:
+        return None
+    vb, xb = {"fp64": (8, 8), "fp32": (4, 4), "bf16": (2, 4)}[precision]
+    constant = all(np.ptp(A.values[d == o - A.nrows]) == 0.0 for o in off)
+    per_row = (1 if len(off) <= 8 else 2) + (0 if constant else vb * len(off))
+    return per_row * A.nrows + xb * (A.ncols + A.nrows)
 
 
 def spmv_bytes(A, precision):
@@ -392,6 +410,9 @@ def run_spmv(args, rank, world, local_rank):
     stream = torch.cuda.current_stream(dev)
     s = stream.cuda_stream
     nbytes = spmv_bytes(A, precision)
+    dia_bytes = (diagonal_form_bytes(A, precision)
+                 if kspmv.tuning(M)["kernel"] == "auto" else None)
+    moved = dia_bytes or nbytes
 
     def step():
         st = lib.nm_spmv(M._h, xd.data_ptr(), yd.data_ptr(), s)
@@ -400,7 +421,7 @@ def run_spmv(args, rank, world, local_rank):
 
     # Operands smaller than L2: flush it between steps (a 256 MB write, outside
     # the per-step events) and time the steps alone.
-    flush = torch.empty(64 << 20, dtype=torch.float32, device=dev) if nbytes < 126e6 else None
+    flush = torch.empty(64 << 20, dtype=torch.float32, device=dev) if moved < 126e6 else None
     for _ in range(args.warmup):
         step()
     torch.cuda.synchronize(dev)
@@ -471,9 +492,9 @@ def run_spmv(args, rank, world, local_rank):
     achieved = nbytes / (kern_avg_ms * 1e-3) / 1e9
     config = spmv_config(desc, args.workload, A, precision)
     config.update({
-        "l2": ("inputs larger than L2 (no flush): %.1f MB per step > 126 MB" % (nbytes / 1e6)
+        "l2": ("inputs larger than L2 (no flush): %.1f MB per step > 126 MB" % (moved / 1e6)
                if flush is None else "inputs smaller than L2 (%.1f MB): L2 flushed (256 MB "
-               "write) between steps, steps timed alone" % (nbytes / 1e6)),
+               "write) between steps, steps timed alone" % (moved / 1e6)),
         "parallelism": f"replicas x{world}", "tuning": tuned,
     })
     if batch:
@@ -485,11 +506,15 @@ def run_spmv(args, rank, world, local_rank):
             "bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
             "frac": round(achieved / peak, 4), "peak_source": peak_src,
             "frac_of_8TBs_spec": round(achieved / 8000.0, 4),
-            "traffic": traffic_for(args.workload),
+            "traffic": None if dia_bytes else traffic_for(args.workload),
             "kernel": ("nm::spmv_gather_kernel (warp per 32 rows, x gathered through L2)"
                        if kspmv.spmv_kernel(M) == "gather"
+                       else "nm::spmv_dia_kernel (diagonal form: fewer bytes than the CSR "
+                            "formula that `achieved` and `value` count)" if dia_bytes
                        else "nm::spmv_kernel (row-block CSR SpMV)"),
             "kernel_avg_us": round(kern_avg_ms * 1e3, 3),
+            "moved_bytes": moved,
+            "moved_frac": round(moved / (kern_avg_ms * 1e-3) / 1e9 / peak, 4),
         },
         "e2e": {
             "value": round(nbytes / (e2e_ms * 1e-3) / 1e9, 2), "unit": "GB/s",
