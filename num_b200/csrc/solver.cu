@@ -1278,7 +1278,7 @@ struct nm_solver {
         bool valid = false;
         int64_t gen = -1;  // lists_gen
         int tiles = 0;     // tile grid
-        int dia = 0;       // grid of bs_spmv_dia
+        int dia = 0;       // bucket of the diagonal form's tiles (0: none)
     };
     StepGraph graphs[8];
     // nm_solver_take_batch: pinned landing of the solutions, slot lists
@@ -1493,8 +1493,14 @@ int tile_bucket(int64_t tiles) {
     return int(std::min<int64_t>(b, INT32_MAX));
 }
 
+// The same for the tiles of systems in diagonal form, 0 without any: what
+// bs_spmv_dia's launch follows.
+int dia_bucket(int64_t tiles) { return tiles > 0 ? tile_bucket(tiles) : 0; }
+
 // bs_spmv_dia's CTAs per tile, as a power of two: enough of them for the GPU,
-// from two (2,048 rows each) to one per row block.
+// from two (2,048 rows each) to one per row block.  The grid does not tell
+// which it was (64 tiles by 8 CTAs, 128 by 4 and 256 by 2 are all 512); the
+// bucket tells both.
 int dia_split(int64_t tiles) {
     int split = 1;
     while (split < 4 && (int64_t(tile_bucket(tiles)) << split) < 512) ++split;
@@ -1502,7 +1508,7 @@ int dia_split(int64_t tiles) {
 }
 
 int dia_grid(int64_t tiles) {
-    return tiles > 0 ? tile_bucket(tiles) << dia_split(tiles) : 0;
+    return dia_bucket(tiles) << dia_split(tiles);
 }
 
 // Grid of a persistent kernel over `count` items (at least one CTA).
@@ -2402,7 +2408,7 @@ extern "C" int nm_solver_step_begin(nm_solver* S, int32_t iters) {
         const bool big = S->h_hdr->bsys > 0;
         const int tiles = tile_bucket(S->h_hdr->itile);
         const bool csr = S->h_hdr->iblk > 0;
-        const int dia = dia_grid(S->h_hdr->dtile);
+        const int dia = dia_bucket(S->h_hdr->dtile);
         auto& G = S->graphs[(csr ? 1 : 0) + (dia ? 2 : 0) + (big ? 4 : 0)];
         if (!G.valid || G.tiles != tiles || G.dia != dia || G.gen != S->lists_gen) {
             S->ctr.graph_captures += 1;
