@@ -48,6 +48,7 @@
 
 #include "cg.cuh"
 #include "spmv.cuh"
+#include "step_lists.cuh"
 
 namespace nm {
 
@@ -588,7 +589,7 @@ __global__ void __launch_bounds__(kThreads)
     const int t = threadIdx.x;
     const int32_t tile = int32_t(blockIdx.x) >> split;
     const int32_t rows = kTileRows >> split;
-    const int4 tl = tiles[tile];
+    const int4 tl = tiles[tile];  // in the list's room (tile_list_room) also past its end
     if (tile >= __ldcg(&hdr->dtile)) return;
     const int32_t slot = tl.z;
     const int32_t row_begin = tl.x + (int32_t(blockIdx.x) - (tile << split)) * rows;
@@ -1354,7 +1355,7 @@ int grow_lists(nm_solver* S, int64_t need_blk, int64_t need_tile) {
         S->cap_blk = c;
     }
     if (need_tile > S->cap_tile) {
-        const int64_t c = std::max<int64_t>(need_tile, 2 * S->cap_tile);
+        const int64_t c = tile_list_room(std::max<int64_t>(need_tile, 2 * S->cap_tile));
         cudaFree(S->itile); cudaFree(S->otile); cudaFree(S->part_tile); cudaFreeHost(S->h_tile);
         S->itile = S->otile = nullptr; S->part_tile = nullptr; S->h_tile = nullptr;
         NM_CUDA_TRY(cudaMalloc(&S->itile, sizeof(int4) * size_t(c)));
@@ -1484,31 +1485,6 @@ CsrView<V> arena_view(const nm_solver* S, const void* values, const BlockDesc* l
     M.stage_x = 1;
     M.nblk_dev = count;
     return M;
-}
-
-// One CTA per tile: the tile count rounded up to a power of two.
-int tile_bucket(int64_t tiles) {
-    int64_t b = 1;
-    while (b < tiles) b <<= 1;
-    return int(std::min<int64_t>(b, INT32_MAX));
-}
-
-// The same for the tiles of systems in diagonal form, 0 without any: what
-// bs_spmv_dia's launch follows.
-int dia_bucket(int64_t tiles) { return tiles > 0 ? tile_bucket(tiles) : 0; }
-
-// bs_spmv_dia's CTAs per tile, as a power of two: enough of them for the GPU,
-// from two (2,048 rows each) to one per row block.  The grid does not tell
-// which it was (64 tiles by 8 CTAs, 128 by 4 and 256 by 2 are all 512); the
-// bucket tells both.
-int dia_split(int64_t tiles) {
-    int split = 1;
-    while (split < 4 && (int64_t(tile_bucket(tiles)) << split) < 512) ++split;
-    return split;
-}
-
-int dia_grid(int64_t tiles) {
-    return dia_bucket(tiles) << dia_split(tiles);
 }
 
 // Grid of a persistent kernel over `count` items (at least one CTA).

@@ -1,6 +1,7 @@
-"""A step's kept graphs against lists that change between steps: large systems
-admitted while others iterate, against the persistent step, which has no graph:
-the same bits and iteration counts."""
+"""A step's graphs against the persistent step, which has none: large systems
+admitted while others iterate, so that the lists change under kept graphs, and
+solvers made for one system, whose lists hold little more than its tiles.  The
+same bits and iteration counts."""
 import numpy as np
 import pytest
 
@@ -55,3 +56,34 @@ def test_diagonal_systems_admitted_between_steps(kspmv, nmlib, before):
     a, b = (_run(nmlib, first, [lap, varcoef, lap], persistent) for persistent in (0, 1))
     for (x, it, res), (y, jt, sres) in zip(a, b):
         assert it == jt and res == sres and np.array_equal(x, y)
+
+
+def _tridiag(n):
+    i = np.arange(n, dtype=np.int64)
+    cols = np.stack([i - 1, i, i + 1], 1)
+    valid = (cols >= 0) & (cols < n)
+    vals = np.stack([np.full(n, -1.0), 2.5 + 0.1 * np.sin(i), np.full(n, -1.0)], 1)
+    rp = np.concatenate([[0], np.cumsum(valid.sum(1))]).astype(np.int32)
+    return gen.Csr(rp, cols[valid].astype(np.int32), vals[valid].copy(), n, n)
+
+
+# 33, 65 and 74 tiles (8 and 4 CTAs to a tile) and 257 and 270 (2 CTAs of 8 row
+# blocks each): the first past a power of two, and one further on
+@pytest.mark.parametrize("n", [131_073, 262_145, 300_008, 1_048_577, 1_104_000])
+def test_solver_made_for_one_system(kspmv, nmlib, n):
+    from num_b200.solver import BatchSolver
+    A = _tridiag(n)
+    b = np.random.default_rng(n).standard_normal(n)
+    out = []
+    for persistent in (0, 1):
+        nmlib.nm_solver_set_persistent(persistent)
+        try:
+            S = BatchSolver(max_rows=n + 8, max_nnz=A.nnz + 32, max_systems=1)
+            s = S.admit(A, b, max_iter=200)
+            while s in S.active:
+                S.step(32)
+            out.append(S.take(s))
+        finally:
+            nmlib.nm_solver_set_persistent(0)
+    (x, i), (y, j) = out
+    assert i["iters"] == j["iters"] and i["residual"] == j["residual"] and np.array_equal(x, y)
