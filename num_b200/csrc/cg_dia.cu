@@ -45,6 +45,7 @@
 
 #include "cg.cuh"
 #include "dia.cuh"
+#include "park_rows.cuh"
 
 namespace nm {
 namespace {
@@ -57,6 +58,7 @@ constexpr size_t kDiaCgMaxSmem = 208 * 1024;
 constexpr int kDiaCgMaxGrid = 160;
 constexpr int kDiaCgSets = 3;  // sets of lines: two of sums in turn, one of flags
 constexpr int kDiaCgLine = 8;  // words of a CTA's line: its tiles, at most 8
+static_assert(kDiaCgTilesPerRow == kDiaCgThreads / kThreads, "tiles of a row of all threads");
 
 struct DiaCgArgs {
     DiaView<double> D;
@@ -174,27 +176,26 @@ __device__ __forceinline__ double wait_word(const ulonglong2* p, ulonglong2 w, u
 
 // Shared memory of the exchanges.
 struct DiaExchange {
-    double scr[28][kWarps];     // this CTA's tiles: a sum per warp
+    double scr[kDiaCgMaxOwnTiles][kWarps];  // this CTA's tiles: a sum per warp
     double sv[kDiaCgTileSums];  // everyone's sums
     double red[kWarps];
     double sc[4];               // what `scalars` leaves
     double rel;                 // the residual the stopping test looks at
 };
 
-// The warp sums of the values of rows q0 .. q0 + N - 1 (N <= 8), parked per
-// tile and warp.
-template <int N>
-__device__ __forceinline__ void park_sums(const double (&d)[8], int q0, double (*scr)[kWarps]) {
-    constexpr int P = N <= 1 ? 1 : (N <= 2 ? 2 : (N <= 4 ? 4 : 8));
-    constexpr int SH = P == 1 ? 5 : (P == 2 ? 4 : (P == 4 ? 3 : 2));
+// The warp sums of the values of the thread's rows q0, q0 + 1, ... (a group of
+// its Q), parked per tile and warp.
+template <int Q>
+__device__ __forceinline__ void park_sums(const double (&d)[kDiaCgGroup], int q0,
+                                          double (*scr)[kWarps]) {
+    static_assert(Q <= kDiaCgMaxQ, "room in scr");
+    constexpr int N = Q < kDiaCgGroup ? Q : kDiaCgGroup, P = park_width(N);
     double v[P];
 #pragma unroll
     for (int q = 0; q < P; ++q) v[q] = q < N ? d[q] : 0.0;
     multi_warp_sum<P>(v);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int q = (lane >> SH) & (P - 1);
-    if ((lane & ((1 << SH) - 1)) == 0 && q < N)
-        scr[(q0 + q) * (kDiaCgThreads / kThreads) + warp / kWarps][warp % kWarps] = v[0];
+    const int warp = threadIdx.x >> 5, row = park_row(threadIdx.x & 31, q0, Q);
+    if (row >= 0) scr[row * kDiaCgTilesPerRow + warp / kWarps][warp % kWarps] = v[0];
 }
 
 // Publishes this CTA's sums (parked in X.scr; the caller has synchronised).
@@ -403,8 +404,8 @@ __global__ void __launch_bounds__(kDiaCgThreads, 1) cg_dia_kernel(const DiaCgArg
         asm volatile("" : "+r"(have), "+r"(shown));
         // ---- Ap = A p (serial CSR-order row sums), p.Ap ----
 #pragma unroll
-        for (int q0 = 0; q0 < Q; q0 += 8) {
-            constexpr int N = 8;
+        for (int q0 = 0; q0 < Q; q0 += kDiaCgGroup) {
+            constexpr int N = kDiaCgGroup;
             double d[N];
 #pragma unroll
             for (int j = 0; j < N; ++j) {
@@ -432,7 +433,7 @@ __global__ void __launch_bounds__(kDiaCgThreads, 1) cg_dia_kernel(const DiaCgArg
                 if (have >> q & 1u) d[j] = fma(pe[own + q * NT + t], acc, 0.0);
                 if (j % 2 == 1) asm volatile("" ::: "memory");  // two rows' loads in flight
             }
-            park_sums<(Q < 8 ? Q : 8)>(d, q0, X.scr);
+            park_sums<Q>(d, q0, X.scr);
         }
         __syncthreads();
         publish<TILES>(a, ++phase, ntile_own, X);
@@ -480,10 +481,10 @@ __global__ void __launch_bounds__(kDiaCgThreads, 1) cg_dia_kernel(const DiaCgArg
         }
         // ---- x += alpha p, r -= alpha Ap, r.r; r to the CTAs that keep the row ----
 #pragma unroll
-        for (int q0 = 0; q0 < Q; q0 += 8) {
-            double d[8];
+        for (int q0 = 0; q0 < Q; q0 += kDiaCgGroup) {
+            double d[kDiaCgGroup];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
+            for (int j = 0; j < kDiaCgGroup; ++j) {
                 d[j] = 0.0;
                 const int q = q0 + j;
                 if (q >= Q) continue;
@@ -497,7 +498,7 @@ __global__ void __launch_bounds__(kDiaCgThreads, 1) cg_dia_kernel(const DiaCgArg
                     d[j] = fma(r[q], r[q], 0.0);
                 }
             }
-            park_sums<(Q < 8 ? Q : 8)>(d, q0, X.scr);
+            park_sums<Q>(d, q0, X.scr);
         }
         __syncthreads();
         publish<TILES>(a, ++phase, ntile_own, X);
