@@ -2,6 +2,7 @@
 #include <algorithm>
 #include <cstring>
 
+#include "batch_shape.cuh"
 #include "dia.cuh"
 
 namespace nm {
@@ -356,10 +357,6 @@ int launch_dia_t(const nm_csr* M, const void* x, void* y, cudaStream_t s) {
 // 320-row runs 442 and 473 us.  What is left waits on X
 // from L2: registers allow 28 of 64 warps per SM, and L1 holds 36 % of the
 // loads.
-constexpr int kDiaBatchThreads = 128;
-constexpr int kDiaBatchCols = 16;
-constexpr int kDiaBatchRun = 192;
-
 template <int KC, bool CONST, int VEC>
 __global__ void __launch_bounds__(kDiaBatchThreads)
     batch_dia_kernel(const DiaView<double> D, int ndiag, int32_t k, int lg, int chunk_cols, int nchunk,
@@ -499,41 +496,27 @@ __global__ void __launch_bounds__(kDiaBatchThreads)
 }
 
 template <int KC, bool CONST, int VEC>
-void launch_batch_dia_t(const nm_csr* A, const double* X, double* Y, int32_t k, cudaStream_t s) {
-    // lanes per row: 16 columns to a chunk, or 8 where that leaves fewer
-    // lanes idle in the last one
-    const int groups = (k + VEC - 1) / VEC;
-    int lg = 0;
-    while ((1 << lg) < groups && (VEC << lg) < kDiaBatchCols) ++lg;
-    auto slots = [&](int l) { return ((groups + (1 << l) - 1) >> l) << l; };
-    if ((1 << lg) < groups && lg > 0 && slots(lg - 1) < slots(lg)) --lg;
-    const int nchunk = (groups + (1 << lg) - 1) >> lg;
-    const int chunk_cols = VEC * ((groups + nchunk - 1) / nchunk);
-    const int step = kDiaBatchThreads >> lg;
-    // Shorter runs where there are too few rows to fill the GPU with them.
-    int64_t run = std::max<int64_t>(step, int64_t(A->nrows) * nchunk / (int64_t(sm_count()) * 16));
-    run = (std::min<int64_t>(run, kDiaBatchRun) + step - 1) / step * step;
-    const int64_t grid = (int64_t(A->nrows) + run - 1) / run * nchunk;
+void launch_batch_dia_t(const nm_csr* A, const DiaBatchShape& b, const double* X, double* Y,
+                        int32_t k, cudaStream_t s) {
     const auto D = dia_view<double>(A->dia, A->nrows);
-    const unsigned g = static_cast<unsigned>(grid);
-    const int32_t r = static_cast<int32_t>(run);
+    const unsigned g = static_cast<unsigned>(b.grid);
     if constexpr (KC > 8)
-        batch_dia_bits_kernel<CONST, VEC><<<g, kDiaBatchThreads, 0, s>>>(D, k, lg, chunk_cols,
-                                                                         nchunk, r, X, Y);
+        batch_dia_bits_kernel<CONST, VEC><<<g, kDiaBatchThreads, 0, s>>>(
+            D, k, b.lg, b.chunk_cols, b.nchunk, b.run, X, Y);
     else
         batch_dia_kernel<KC, CONST, VEC><<<g, kDiaBatchThreads, 0, s>>>(
-            D, A->dia.ndiag, k, lg, chunk_cols, nchunk, r, X, Y);
+            D, A->dia.ndiag, k, b.lg, b.chunk_cols, b.nchunk, b.run, X, Y);
 }
 
 template <int KC>
-void launch_batch_dia_k(const nm_csr* A, const double* X, double* Y, int32_t k, bool vec2,
-                        cudaStream_t s) {
+void launch_batch_dia_k(const nm_csr* A, const DiaBatchShape& b, const double* X, double* Y,
+                        int32_t k, bool vec2, cudaStream_t s) {
     if (A->dia.constant) {
-        if (vec2) launch_batch_dia_t<KC, true, 2>(A, X, Y, k, s);
-        else launch_batch_dia_t<KC, true, 1>(A, X, Y, k, s);
+        if (vec2) launch_batch_dia_t<KC, true, 2>(A, b, X, Y, k, s);
+        else launch_batch_dia_t<KC, true, 1>(A, b, X, Y, k, s);
     } else {
-        if (vec2) launch_batch_dia_t<KC, false, 2>(A, X, Y, k, s);
-        else launch_batch_dia_t<KC, false, 1>(A, X, Y, k, s);
+        if (vec2) launch_batch_dia_t<KC, false, 2>(A, b, X, Y, k, s);
+        else launch_batch_dia_t<KC, false, 1>(A, b, X, Y, k, s);
     }
 }
 
@@ -576,11 +559,13 @@ int launch_spmv_dia(const nm_csr* A, const void* x, void* y, cudaStream_t s) {
 int launch_batch_dia(const nm_csr* A, const double* X, double* Y, int32_t k, bool vec2,
                      cudaStream_t s) {
     const int nd = A->dia.ndiag;
-    if (nd <= 3) launch_batch_dia_k<3>(A, X, Y, k, vec2, s);
-    else if (nd <= 5) launch_batch_dia_k<5>(A, X, Y, k, vec2, s);
-    else if (nd <= 7) launch_batch_dia_k<7>(A, X, Y, k, vec2, s);
-    else if (nd <= 8) launch_batch_dia_k<8>(A, X, Y, k, vec2, s);
-    else launch_batch_dia_k<kDiaMax>(A, X, Y, k, vec2, s);
+    const DiaBatchShape b = dia_batch_shape(A->nrows, k, vec2 ? 2 : 1, sm_count());
+    if (b.grid > INT32_MAX) return fail(NM_ERR_INVALID, "batch_spmv: problem too large");
+    if (nd <= 3) launch_batch_dia_k<3>(A, b, X, Y, k, vec2, s);
+    else if (nd <= 5) launch_batch_dia_k<5>(A, b, X, Y, k, vec2, s);
+    else if (nd <= 7) launch_batch_dia_k<7>(A, b, X, Y, k, vec2, s);
+    else if (nd <= 8) launch_batch_dia_k<8>(A, b, X, Y, k, vec2, s);
+    else launch_batch_dia_k<kDiaMax>(A, b, X, Y, k, vec2, s);
     NM_CHECK_LAUNCH();
     return NM_OK;
 }
