@@ -157,34 +157,61 @@ int validate_csr(const int32_t* rp, const int32_t* ci, int32_t nrows, int32_t nc
     return NM_OK;
 }
 
-// The row offsets (rp_len of them) and, behind them, room for the search for a
-// diagonal form and for its masks: one allocation.
-int alloc_row_ptr(nm_csr* A, size_t rp_len) {
-    const size_t rb = (sizeof(int32_t) * rp_len + 255) & ~size_t(255);
-    NM_CUDA_TRY(cudaMalloc(&A->d_row_ptr, rb + kDiaTableBytes + 2 * size_t(A->nrows) + 256));
-    A->d_dia_room = reinterpret_cast<unsigned char*>(A->d_row_ptr) + rb;
+// The matrix's arrays (rp_len row offsets, nnz_pad columns and values) and,
+// where it may have a diagonal form, room for the search for it and for its
+// masks: one allocation.
+int alloc_arrays(nm_csr* A, size_t rp_len, size_t nnz_pad, bool dia_room) {
+    auto up = [](size_t b) { return (b + 255) & ~size_t(255); };
+    const size_t rb = up(sizeof(int32_t) * rp_len), cb = up(sizeof(int32_t) * nnz_pad);
+    const size_t vb = up(dtype_size(A->dtype) * nnz_pad);
+    const size_t db = dia_room ? kDiaTableBytes + 2 * size_t(A->nrows) : 0;
+    unsigned char* base = nullptr;
+    NM_CUDA_TRY(cudaMalloc(&base, rb + cb + vb + db));
+    A->d_row_ptr = reinterpret_cast<int32_t*>(base);
+    A->d_col_idx = reinterpret_cast<int32_t*>(base + rb);
+    A->d_values = base + rb + cb;
+    A->d_dia_room = dia_room ? base + rb + cb + vb : nullptr;
     return NM_OK;
 }
+
+// Arrays of up to this many bytes go up in one copy out of a host image of
+// their allocation, instead of a copy and a clearing of the padding each: with
+// the search under the row blocks (finish_create) that pays for the search
+// (16^2 and 64^2 Laplacian: 403 and 463 us, 440 and 492 with neither, 406 and
+// 461 without a search).
+constexpr size_t kImageBytes = size_t(512) << 10;
 
 int upload(nm_csr* A, const int32_t* rp, const int32_t* ci, const void* vals) {
     const size_t es = dtype_size(A->dtype);
     const int64_t nnz_pad = ((static_cast<int64_t>(A->nnz) + 7) & ~int64_t(7)) + 8;
     const size_t rp_len = size_t(A->nrows) + 1 + 8;
-    const int st = alloc_row_ptr(A, rp_len);
+    const int st = alloc_arrays(A, rp_len, size_t(nnz_pad), may_be_diagonal(rp, ci, A->nrows));
     if (st != NM_OK) return st;
-    NM_CUDA_TRY(cudaMalloc(&A->d_col_idx, sizeof(int32_t) * size_t(nnz_pad)));
-    NM_CUDA_TRY(cudaMalloc(&A->d_values, es * size_t(nnz_pad)));
+    const size_t rb = sizeof(int32_t) * rp_len, nzb = sizeof(int32_t) * size_t(A->nnz);
+    unsigned char* base = reinterpret_cast<unsigned char*>(A->d_row_ptr);
+    const size_t col_at = size_t(reinterpret_cast<unsigned char*>(A->d_col_idx) - base);
+    const size_t val_at = size_t(static_cast<unsigned char*>(A->d_values) - base);
+    const size_t image = val_at + es * size_t(nnz_pad);
+    if (image <= kImageBytes) {
+        std::vector<unsigned char> h(image);
+        std::memcpy(h.data(), rp, sizeof(int32_t) * (size_t(A->nrows) + 1));
+        std::fill_n(reinterpret_cast<int32_t*>(h.data()) + A->nrows + 1, 8, rp[A->nrows]);
+        if (A->nnz > 0) {
+            std::memcpy(h.data() + col_at, ci, nzb);
+            std::memcpy(h.data() + val_at, vals, es * size_t(A->nnz));
+        }
+        NM_CUDA_TRY(cudaMemcpy(base, h.data(), image, cudaMemcpyHostToDevice));
+        return NM_OK;
+    }
     {
         std::vector<int32_t> rpp(rp, rp + A->nrows + 1);
         rpp.resize(rp_len, rp[A->nrows]);
-        NM_CUDA_TRY(cudaMemcpy(A->d_row_ptr, rpp.data(), sizeof(int32_t) * rp_len,
-                               cudaMemcpyHostToDevice));
+        NM_CUDA_TRY(cudaMemcpy(A->d_row_ptr, rpp.data(), rb, cudaMemcpyHostToDevice));
     }
     NM_CUDA_TRY(cudaMemset(A->d_col_idx, 0, sizeof(int32_t) * size_t(nnz_pad)));
     NM_CUDA_TRY(cudaMemset(A->d_values, 0, es * size_t(nnz_pad)));
     if (A->nnz > 0) {
-        NM_CUDA_TRY(cudaMemcpy(A->d_col_idx, ci, sizeof(int32_t) * size_t(A->nnz),
-                               cudaMemcpyHostToDevice));
+        NM_CUDA_TRY(cudaMemcpy(A->d_col_idx, ci, nzb, cudaMemcpyHostToDevice));
         NM_CUDA_TRY(cudaMemcpy(A->d_values, vals, es * size_t(A->nnz), cudaMemcpyHostToDevice));
     }
     return NM_OK;
@@ -278,8 +305,9 @@ int finish_create(nm_csr* A, const int32_t* rp, const int32_t* ci, const void* v
     if (st == NM_OK) {
         A->h_row_ptr.assign(rp, rp + A->nrows + 1);
         A->h_col_idx.assign(ci, ci + A->nnz);
-        st = rebuild_blocks(A);
-        if (st == NM_OK) st = find_dia_form(A);
+        st = search_dia_form(A);
+        if (st == NM_OK) st = rebuild_blocks(A);
+        if (st == NM_OK) st = take_dia_form(A);
     }
     if (st != NM_OK) {
         delete A;
@@ -308,9 +336,7 @@ int spmv_grid(const nm_csr* A, int ctas_per_sm) {
 nm_csr::~nm_csr() {
     cg.reset();
     host_spmv.reset();
-    if (d_row_ptr) cudaFree(d_row_ptr);
-    if (d_col_idx) cudaFree(d_col_idx);
-    if (d_values) cudaFree(d_values);
+    if (d_row_ptr) cudaFree(d_row_ptr);  // and the columns, values and d_dia_room behind it
     if (d_desc) cudaFree(d_desc);  // and d_blk behind it
     if (d_sell_ptr) cudaFree(d_sell_ptr);
     if (d_sell_row) cudaFree(d_sell_row);
@@ -410,8 +436,8 @@ extern "C" int nm_csr_laplacian(int32_t dim, int32_t L, int dtype, nm_csr** out)
     if (dim != 2 && dim != 3)
         return fail(NM_ERR_INVALID, "nm_csr_laplacian: dim must be 2 or 3 (got %d)", dim);
     if (L <= 0) return fail(NM_ERR_INVALID, "CrsMatrixHandle: non-positive dimensions");
-    const size_t es = nm::dtype_size(dtype);
-    if (es == 0) return fail(NM_ERR_TYPE, "nm_csr_laplacian: unknown dtype %d", dtype);
+    if (nm::dtype_size(dtype) == 0)
+        return fail(NM_ERR_TYPE, "nm_csr_laplacian: unknown dtype %d", dtype);
     // L^dim rows and their nonzeros must fit the int32 offsets (checked in
     // 64 bits; L above 46,341 / 1,291 already overflows the rows).
     if ((dim == 2 && L > 46341) || (dim == 3 && L > 1291))
@@ -433,15 +459,10 @@ extern "C" int nm_csr_laplacian(int32_t dim, int32_t L, int dtype, nm_csr** out)
         // Same allocation and padding as an uploaded matrix.
         const int64_t nnz_pad = ((nnz + 7) & ~int64_t(7)) + 8;
         const int64_t rp_len = n + 1 + 8;
-        int st = nm::alloc_row_ptr(A, size_t(rp_len));
+        int st = nm::alloc_arrays(A, size_t(rp_len), size_t(nnz_pad), true);
         if (st != NM_OK) return st;
-        NM_CUDA_TRY(cudaMalloc(&A->d_col_idx, sizeof(int32_t) * size_t(nnz_pad)));
-        NM_CUDA_TRY(cudaMalloc(&A->d_values, es * size_t(nnz_pad)));
-        NM_CUDA_TRY(cudaMemset(A->d_col_idx + nnz, 0, sizeof(int32_t) * size_t(nnz_pad - nnz)));
-        NM_CUDA_TRY(cudaMemset(static_cast<char*>(A->d_values) + es * size_t(nnz), 0,
-                               es * size_t(nnz_pad - nnz)));
         st = nm::launch_laplacian(dim, L, dtype, A->d_row_ptr, rp_len, A->d_col_idx,
-                                      A->d_values, nullptr);
+                                  A->d_values, nnz_pad, nullptr);
         if (st != NM_OK) return st;
         // The row-block partition is built on the host from row_ptr and the
         // columns (as for an uploaded matrix): read them back once.
@@ -451,8 +472,9 @@ extern "C" int nm_csr_laplacian(int32_t dim, int32_t L, int dtype, nm_csr** out)
                                cudaMemcpyDeviceToHost));
         NM_CUDA_TRY(cudaMemcpy(A->h_col_idx.data(), A->d_col_idx, sizeof(int32_t) * size_t(nnz),
                                cudaMemcpyDeviceToHost));
-        st = nm::rebuild_blocks(A);
-        return st == NM_OK ? nm::find_dia_form(A) : st;
+        st = nm::search_dia_form(A);
+        if (st == NM_OK) st = nm::rebuild_blocks(A);
+        return st == NM_OK ? nm::take_dia_form(A) : st;
     };
     const int st = build();
     if (st != NM_OK) {

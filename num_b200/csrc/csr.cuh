@@ -1,12 +1,13 @@
 // csr.cuh -- internal layout of a device CSR matrix.
 //
-// HBM layout (one cudaMalloc each, 256-byte aligned):
-//   row_ptr  int32[nrows + 1 + 8]  pad = nnz; behind it the room of DiaForm
+// HBM layout (256-byte aligned), two allocations: the first three with the room
+// of DiaForm behind them, and the last two (32^3 varying coefficients, upload:
+// 1.74 ms, 2.06 with the first three apart):
+//   row_ptr  int32[nrows + 1 + 8]  pad = nnz
 //   col_idx  int32[nnz_pad]        nnz_pad = round_up(nnz, 8) + 8, pad = column 0
 //   values   V[nnz_pad]            pad = 0
 //   desc     BlockDesc[nblk]       per block rows, nonzeros and x windows
-//   blk      int32[nblk + 1]       row-block boundaries (see build_row_blocks),
-//                                  behind desc
+//   blk      int32[nblk + 1]       row-block boundaries (see build_row_blocks)
 // The padding lets the TMA bulk copies of a block start and end on 16-byte
 // boundaries (nonzeros rounded to multiples of 8, row_ptr to multiples of 4),
 // and lets a thread load 4 consecutive nonzeros with one 16-byte access,
@@ -74,7 +75,7 @@ struct DiaForm {
     void* d_val = nullptr;   // values [ndiag][ld], the matrix's type
 };
 
-// Room behind the row offsets for the search for that form (dia.cu); the masks
+// Room behind the values for the search for that form (dia.cu); the masks
 // follow it there.
 constexpr size_t kDiaTableBytes = 512;
 
@@ -158,7 +159,7 @@ struct nm_csr {
     void* d_sell_val = nullptr;
     // The matrix in diagonal form, when its nonzeros lie on few diagonals
     // (found once, when the arrays are in place); d_dia_room lies behind the
-    // row offsets in their allocation.
+    // values in their allocation (null where may_be_diagonal said no).
     nm::DiaForm dia;
     unsigned char* d_dia_room = nullptr;
     // The plain SpMV runs on the diagonal form: it sums every row by one
@@ -207,9 +208,13 @@ constexpr int32_t kSellWindow = 65536;
 // Builds A's sliced copy for the gather kernel once (spmv.cu); NM_OK also
 // when the layout would pad too much (A->sell_ready stays false).
 int build_sell(nm_csr* A);
-// Looks for A's diagonal form (dia.cu) once its arrays are on the device;
-// NM_OK also when it has none.
-int find_dia_form(nm_csr* A);
+// Whether a look at some rows leaves room for a diagonal form (dia.cu).
+bool may_be_diagonal(const int32_t* row_ptr, const int32_t* col_idx, int32_t nrows);
+// Looks for A's diagonal form (dia.cu) once its arrays are on the device: the
+// search is started, and its result taken after the host's work on the row
+// blocks, under which it runs.  NM_OK also when A has none.
+int search_dia_form(const nm_csr* A);
+int take_dia_form(nm_csr* A);
 // y = A x on the diagonal form.
 int launch_spmv_dia(const nm_csr* A, const void* x, void* y, cudaStream_t stream);
 // Y = A X (row-major, k columns; vec2: k even and X, Y 16-byte aligned) on the
@@ -221,7 +226,8 @@ void reset_cg(nm_csr* A);
 // Nonzeros of the Laplacian on an L^dim grid (dim 2: 5-point, dim 3: 7-point).
 int64_t stencil_nnz(int dim, int32_t L);
 // Writes that Laplacian's row_ptr (rp_len entries, those past the last row =
-// nnz), col_idx and values (dtype) into device arrays on `stream` (gen.cu).
+// nnz), col_idx and values (dtype; nnz_pad entries each, those past nnz = 0)
+// into device arrays on `stream` (gen.cu).
 int launch_laplacian(int dim, int32_t L, int dtype, int32_t* rp, int64_t rp_len, int32_t* ci,
-                     void* val, cudaStream_t stream);
+                     void* val, int64_t nnz_pad, cudaStream_t stream);
 }  // namespace nm

@@ -9,7 +9,7 @@ namespace nm {
 
 namespace {
 
-// What the search kernel finds, in device memory behind the row offsets.
+// What the search kernel finds, in device memory (nm_csr::d_dia_room).
 constexpr int kDiaSlots = kDiaMax + 1;         // one more than allowed: overflow
 constexpr int32_t kDiaNoOff = INT32_MIN;       // col - row is never this
 constexpr uint64_t kDiaNoVal = 0x7FF0D1A0D1A0D1A0ull;  // a signalling NaN
@@ -147,16 +147,25 @@ __global__ void __launch_bounds__(kThreads)
     if ((threadIdx.x & 31) == 0 && any) atomicAdd(&T->pairs, static_cast<unsigned long long>(__popc(any)));
 }
 
+int64_t row_ctas(const nm_csr* A) { return (int64_t(A->nrows) + kThreads - 1) / kThreads; }
+
 template <typename V>
-int find_form(nm_csr* A, const DiaSeed& seed) {
+int launch_search(const nm_csr* A, const DiaSeed& seed) {
+    DiaTable* T = reinterpret_cast<DiaTable*>(A->d_dia_room);
+    const V* vals = static_cast<const V*>(A->d_values);
+    dia_seed_kernel<V><<<1, 32>>>(seed, vals, T);
+    dia_find_kernel<V><<<static_cast<int>(std::min<int64_t>(row_ctas(A), int64_t(sm_count()) * 8)),
+                         kThreads>>>(A->d_row_ptr, A->d_col_idx, vals, A->nrows, T);
+    NM_CHECK_LAUNCH();
+    return NM_OK;
+}
+
+template <typename V>
+int take_form(nm_csr* A) {
     DiaTable* T = reinterpret_cast<DiaTable*>(A->d_dia_room);
     const V* vals = static_cast<const V*>(A->d_values);
     const int32_t n = A->nrows;
-    dia_seed_kernel<V><<<1, 32>>>(seed, vals, T);
-    const int64_t want = (int64_t(n) + kThreads - 1) / kThreads;
-    dia_find_kernel<V><<<static_cast<int>(std::min<int64_t>(want, int64_t(sm_count()) * 8)),
-                         kThreads>>>(A->d_row_ptr, A->d_col_idx, vals, n, T);
-    NM_CHECK_LAUNCH();
+    const int64_t want = row_ctas(A);
     DiaTable h;
     NM_CUDA_TRY(cudaMemcpy(&h, T, sizeof h, cudaMemcpyDeviceToHost));
     if (h.overflow || h.disorder) return NM_OK;
@@ -520,31 +529,50 @@ void launch_batch_dia_k(const nm_csr* A, const DiaBatchShape& b, const double* X
     }
 }
 
-}  // namespace
-
-int find_dia_form(nm_csr* A) {
-    if (A->nnz == 0 || A->nrows == 0) return NM_OK;
-    // A look at some rows on the host first: a matrix of scattered columns
-    // shows more than kDiaMax offsets there and costs nothing more.
-    const int32_t* rp = A->h_row_ptr.data();
-    const int32_t* ci = A->h_col_idx.data();
-    DiaSeed seed{};
+// The diagonals of some rows, on the host: a matrix of scattered columns shows
+// more than kDiaMax there (false) and costs nothing more.
+bool look_at_rows(const int32_t* rp, const int32_t* ci, int32_t nrows, DiaSeed* seed) {
+    if (nrows == 0 || rp[nrows] == 0) return false;
     constexpr int kLook = 64;
     for (int q = 0; q < kLook; ++q) {
-        const int32_t r = static_cast<int32_t>(int64_t(A->nrows - 1) * q / (kLook - 1));
-        if (rp[r + 1] - rp[r] > kDiaMax) return NM_OK;
+        const int32_t r = static_cast<int32_t>(int64_t(nrows - 1) * q / (kLook - 1));
+        if (rp[r + 1] - rp[r] > kDiaMax) return false;
         for (int32_t z = rp[r]; z < rp[r + 1]; ++z) {
             const int32_t d = ci[z] - r;
-            if (std::find(seed.off, seed.off + seed.count, d) != seed.off + seed.count) continue;
-            if (seed.count == kDiaMax) return NM_OK;
-            seed.off[seed.count] = d;
-            seed.at[seed.count++] = z;
+            if (std::find(seed->off, seed->off + seed->count, d) != seed->off + seed->count)
+                continue;
+            if (seed->count == kDiaMax) return false;
+            seed->off[seed->count] = d;
+            seed->at[seed->count++] = z;
         }
     }
+    return true;
+}
+
+}  // namespace
+
+bool may_be_diagonal(const int32_t* row_ptr, const int32_t* col_idx, int32_t nrows) {
+    DiaSeed seed{};
+    return look_at_rows(row_ptr, col_idx, nrows, &seed);
+}
+
+int search_dia_form(const nm_csr* A) {
+    if (!A->d_dia_room) return NM_OK;
+    DiaSeed seed{};
+    look_at_rows(A->h_row_ptr.data(), A->h_col_idx.data(), A->nrows, &seed);
     switch (A->dtype) {
-        case NM_F64: return find_form<double>(A, seed);
-        case NM_F32: return find_form<float>(A, seed);
-        default: return find_form<__nv_bfloat16>(A, seed);
+        case NM_F64: return launch_search<double>(A, seed);
+        case NM_F32: return launch_search<float>(A, seed);
+        default: return launch_search<__nv_bfloat16>(A, seed);
+    }
+}
+
+int take_dia_form(nm_csr* A) {
+    if (!A->d_dia_room) return NM_OK;
+    switch (A->dtype) {
+        case NM_F64: return take_form<double>(A);
+        case NM_F32: return take_form<float>(A);
+        default: return take_form<__nv_bfloat16>(A);
     }
 }
 

@@ -48,14 +48,15 @@ namespace {
 // stages the row's nonzeros in shared memory at their offset within the
 // group; the CTA then writes the group's contiguous column / value range with
 // consecutive threads on consecutive elements (full-sector stores), and CTA 0
-// fills the row_ptr padding past row n - 1 with nnz.
+// fills the row_ptr padding past row n - 1 with nnz and the columns and values
+// past nnz with zeros.
 constexpr int kGenRows = 256;
 constexpr int kGenMaxNz = 7;  // nonzeros of a 7-point row
 
 template <typename V>
 __global__ void __launch_bounds__(kGenRows)
     laplacian_kernel(int dim, uint32_t L, uint32_t n, int64_t rp_len, int32_t* __restrict__ rp,
-                     int32_t* __restrict__ ci, V* __restrict__ val, V diag, V off) {
+                     int32_t* __restrict__ ci, V* __restrict__ val, int64_t nnz_pad, V diag, V off) {
     __shared__ int32_t s_ci[kGenRows * kGenMaxNz];
     __shared__ V s_v[kGenRows * kGenMaxNz];
     const uint32_t LL = L * L;
@@ -88,19 +89,28 @@ __global__ void __launch_bounds__(kGenRows)
         }
         __syncthreads();
     }
-    if (blockIdx.x == 0 && int64_t(n) + threadIdx.x < rp_len)
-        rp[int64_t(n) + threadIdx.x] = static_cast<int32_t>(stencil_before(dim, L, n, n));
+    if (blockIdx.x == 0) {
+        const int64_t nnz = stencil_before(dim, L, n, n);
+        if (int64_t(n) + threadIdx.x < rp_len)
+            rp[int64_t(n) + threadIdx.x] = static_cast<int32_t>(nnz);
+        if (nnz + threadIdx.x < nnz_pad) {
+            ci[nnz + threadIdx.x] = 0;
+            val[nnz + threadIdx.x] = V(0.0f);
+        }
+    }
 }
 
 template <typename V>
 int launch_t(int dim, int32_t L, int32_t n, int64_t rp_len, int32_t* rp, int32_t* ci, void* val,
-             V diag, V off, cudaStream_t s) {
+             int64_t nnz_pad, V diag, V off, cudaStream_t s) {
     if (rp_len < int64_t(n) + 1 || rp_len - n > kGenRows)
         return fail(NM_ERR_INVALID, "laplacian: row_ptr length %lld for %d rows", (long long)rp_len, n);
+    if (nnz_pad - stencil_nnz(dim, L) > kGenRows)
+        return fail(NM_ERR_INVALID, "laplacian: too much padding");
     const int64_t blocks =
         std::min<int64_t>((int64_t(n) + kGenRows - 1) / kGenRows, int64_t(sm_count()) * 8);
     laplacian_kernel<V><<<static_cast<int>(blocks), kGenRows, 0, s>>>(
-        dim, uint32_t(L), uint32_t(n), rp_len, rp, ci, static_cast<V*>(val), diag, off);
+        dim, uint32_t(L), uint32_t(n), rp_len, rp, ci, static_cast<V*>(val), nnz_pad, diag, off);
     NM_CHECK_LAUNCH();
     return NM_OK;
 }
@@ -108,15 +118,15 @@ int launch_t(int dim, int32_t L, int32_t n, int64_t rp_len, int32_t* rp, int32_t
 }  // namespace
 
 int launch_laplacian(int dim, int32_t L, int dtype, int32_t* rp, int64_t rp_len, int32_t* ci,
-                     void* val, cudaStream_t s) {
+                     void* val, int64_t nnz_pad, cudaStream_t s) {
     const int32_t n = dim == 2 ? L * L : L * L * L;
     const double d = dim == 2 ? 4.0 : 6.0;
     switch (dtype) {
-        case NM_F64: return launch_t<double>(dim, L, n, rp_len, rp, ci, val, d, -1.0, s);
+        case NM_F64: return launch_t<double>(dim, L, n, rp_len, rp, ci, val, nnz_pad, d, -1.0, s);
         case NM_F32:
-            return launch_t<float>(dim, L, n, rp_len, rp, ci, val, float(d), -1.0f, s);
+            return launch_t<float>(dim, L, n, rp_len, rp, ci, val, nnz_pad, float(d), -1.0f, s);
         case NM_BF16:
-            return launch_t<__nv_bfloat16>(dim, L, n, rp_len, rp, ci, val,
+            return launch_t<__nv_bfloat16>(dim, L, n, rp_len, rp, ci, val, nnz_pad,
                                            __float2bfloat16_rn(float(d)),
                                            __float2bfloat16_rn(-1.0f), s);
         default: return fail(NM_ERR_TYPE, "laplacian: unknown dtype %d", dtype);
