@@ -64,7 +64,9 @@ typedef struct {
  * AUTO: a matrix whose nonzeros lie on at most 16 diagonals (rows ascending,
  * none longer than short_max) runs from its diagonal form -- masks and values
  * by diagonal, no column indices -- with the sums of BLOCKS bit for bit, and is
- * reported as BLOCKS; else GATHER when at least 3/4 of the nonzeros lie in row blocks without x
+ * reported as BLOCKS (values that vary along a diagonal are held a second time
+ * for it, if that copy takes at most 64 MB or a quarter of the free device
+ * memory); else GATHER when at least 3/4 of the nonzeros lie in row blocks without x
  * windows and no row has more than 4096 nonzeros, else BLOCKS.  The
  * autotuner times all three.  CG and the batched engine always use the
  * row-block pipeline. */

@@ -86,6 +86,21 @@ int kernel_occupancy(const void* fn, int threads, int* ctas_per_sm) {
     return NM_OK;
 }
 
+bool alloc_copy(void** out, size_t bytes) {
+    *out = nullptr;
+    if (bytes > kCopyAlways) {
+        size_t free_bytes = 0, total = 0;
+        if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess || bytes > free_bytes / 4) {
+            cudaGetLastError();
+            return false;
+        }
+    }
+    if (cudaMalloc(out, bytes) == cudaSuccess) return true;
+    cudaGetLastError();
+    *out = nullptr;
+    return false;
+}
+
 namespace {
 std::mutex g_err_mu;
 std::unordered_map<int, std::pair<unsigned int*, unsigned int*>> g_err;  // dev -> (host, device)

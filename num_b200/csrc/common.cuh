@@ -40,6 +40,14 @@ int prepare_kernel(const void* fn, int threads, size_t smem, int* ctas_per_sm);
 // memory (once per device; its attributes are left alone).
 int kernel_occupancy(const void* fn, int threads, int* ctas_per_sm);
 
+// Device memory for a second copy of values that another array holds already
+// (the diagonal form's): false, and nothing allocated, where it would take more
+// than a quarter of the memory that is free, so that programs which fill the
+// device keep their room.  Copies up to kCopyAlways are not asked about
+// (cudaMemGetInfo takes longer than uploading them).
+constexpr size_t kCopyAlways = size_t(64) << 20;
+bool alloc_copy(void** out, size_t bytes);
+
 // Device error codes.
 constexpr unsigned int kErrWaitTimeout = 1u;  // a bounded mbarrier wait gave up
 

@@ -194,11 +194,8 @@ int take_form(nm_csr* A) {
         }
     }
     f.d_mask = A->d_dia_room + kDiaTableBytes;
-    if (!constant &&
-        cudaMalloc(&f.d_val, sizeof(V) * size_t(nd) * size_t(f.ld)) != cudaSuccess) {
-        cudaGetLastError();  // no room beside the CSR arrays: they serve alone
-        return NM_OK;
-    }
+    if (!constant && !alloc_copy(&f.d_val, sizeof(V) * size_t(nd) * size_t(f.ld)))
+        return NM_OK;  // no room beside the CSR arrays: they serve alone
     if (nd <= 8)
         dia_fill_kernel<V, uint8_t><<<static_cast<int>(want), kThreads>>>(
             A->d_row_ptr, A->d_col_idx, vals, n, o, static_cast<uint8_t*>(f.d_mask),

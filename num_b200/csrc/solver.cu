@@ -2129,12 +2129,9 @@ int64_t dia_value_room(nm_solver* S, int64_t count) {
     if (!S->dv_tried) {
         S->dv_tried = true;
         const int64_t cap = S->cap_nnz + S->cap_nnz / 8 + 64;
-        if (cudaMalloc(&S->dv, inner_val_bytes(S->inner) * size_t(cap)) == cudaSuccess) {
+        if (alloc_copy(&S->dv, inner_val_bytes(S->inner) * size_t(cap))) {
             S->dvals.init(cap);
             for (auto& g : S->graphs) g.valid = false;  // they hold the pointer
-        } else {
-            cudaGetLastError();
-            S->dv = nullptr;
         }
     }
     return S->dv ? S->dvals.alloc(count) : -1;

@@ -27,9 +27,11 @@ PHASE_REFINE, PHASE_ITERATE, PHASE_DONE = 1, 2, 3
 
 
 def arena_bytes(max_rows: int, max_nnz: int, precision: str = "fp32") -> int:
-    """Device bytes a solver with these capacities allocates when created (the
-    first system on few diagonals whose values vary along them makes it
-    allocate 9/8 max_nnz inner values more, where there is room)."""
+    """Device bytes a solver with these capacities allocates when created.  The
+    first large system on few diagonals whose values vary along them makes it
+    allocate 9/8 max_nnz inner values more (what arena_for sizes stays within
+    its budget with them), unless they are above 64 MB and more than a quarter
+    of the memory that is free then: such systems run from their CSR arrays."""
     t = 8 if precision == "fp64" else 4
     v = {"fp64": 0, "fp32": 4, "bf16": 2}[precision]
     return (max_rows + 16) * (4 + 1 + 3 * 8 + 6 * t) + (max_nnz + 16) * (4 + 8 + v)
