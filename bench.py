@@ -73,8 +73,8 @@ WORKLOADS = {
                       "FP64", "batch", "fp64"),
     "cg_c1": ("2-D 5-point Laplacian 256^2, plain FP64 CG, b = A*1, x0 = 0, tol 1e-8", "cg",
               "fp64"),
-    "cg_1m": ("2-D 5-point Laplacian 1024^2 (1,048,576 rows: the CUDA-graph path), plain FP64 "
-              "CG, b = A*1, x0 = 0, tol 1e-8", "cg", "fp64"),
+    "cg_1m": ("2-D 5-point Laplacian 1024^2 (1,048,576 rows), plain FP64 CG, "
+              "b = A*1, x0 = 0, tol 1e-8", "cg", "fp64"),
     "vec_c2a": ("CG vector ops at 4,096,000 elements: axpy, axpy2 and dot per step", "vec",
                 "fp64"),
     "halo_c2a": ("halo pack + unpack of the 160^3 Laplacian split into 8 row slabs (8 virtual "
@@ -173,21 +173,17 @@ def block_diagonal(mats):
                np.concatenate(vals), r, r)
 
 
-def diagonal_form_bytes(A, precision):
-    """Bytes one SpMV moves when A is stored in diagonal form (at most 16
-    diagonals): masks, the values by diagonal unless each is one number, x and
-    y.  None for other matrices."""
-    row = np.repeat(np.arange(A.nrows, dtype=np.int64), np.diff(A.row_ptr))
-    d = A.col_idx - row
-    if len(np.unique(d[:4096])) > 16 or len(np.unique(d[-4096:])) > 16:
+def diagonal_form_bytes(M, precision):
+    """Bytes one SpMV moves when the library runs M from its diagonal form:
+    what it reads of the matrix, x and y.  None where it does not."""
+    import ctypes as C
+
+    from num_b200 import _lib
+    nd, matrix = C.c_int32(), C.c_int64()
+    _lib.check(_lib.load().nm_csr_diagonals(M._h, C.byref(nd), C.byref(matrix)))
+    if nd.value == 0:
         return None
-    off = np.flatnonzero(np.bincount(d + A.nrows))
-    if len(off) > 16:
-        return None
-    vb, xb = {"fp64": (8, 8), "fp32": (4, 4), "bf16": (2, 4)}[precision]
-    constant = all(np.ptp(A.values[d == o - A.nrows]) == 0.0 for o in off)
-    per_row = (1 if len(off) <= 8 else 2) + (0 if constant else vb * len(off))
-    return per_row * A.nrows + xb * (A.ncols + A.nrows)
+    return matrix.value + (8 if precision == "fp64" else 4) * (M.ncols + M.nrows)
 
 
 def spmv_bytes(A, precision):
@@ -212,6 +208,12 @@ def engine_iter_bytes(nnz, n, vb, tb):
     columns + row_ptr, p gathered once, Ap written); update (p, Ap, r, d,
     D^-1 read; d, r, z written); p update (z, p read; p written)."""
     return (vb + 4) * nnz + 4 * (n + 1) + 13 * tb * n
+
+
+def engine_iter_bytes_dia(nnz, n, vb, tb):
+    """The same for a large system in diagonal form whose values vary: its
+    SpMV reads the values and a mask byte per row."""
+    return vb * nnz + n + 13 * tb * n
 
 
 def engine_outer_bytes(nnz, n, tb):
@@ -410,8 +412,7 @@ def run_spmv(args, rank, world, local_rank):
     stream = torch.cuda.current_stream(dev)
     s = stream.cuda_stream
     nbytes = spmv_bytes(A, precision)
-    dia_bytes = (diagonal_form_bytes(A, precision)
-                 if kspmv.tuning(M)["kernel"] == "auto" else None)
+    dia_bytes = diagonal_form_bytes(M, precision)
     moved = dia_bytes or nbytes
 
     def step():
@@ -489,7 +490,7 @@ def run_spmv(args, rank, world, local_rank):
     if rank != 0:
         return None
     peak, peak_src = measured_peak()
-    achieved = nbytes / (kern_avg_ms * 1e-3) / 1e9
+    achieved = moved / (kern_avg_ms * 1e-3) / 1e9
     config = spmv_config(desc, args.workload, A, precision)
     config.update({
         "l2": ("inputs larger than L2 (no flush): %.1f MB per step > 126 MB" % (moved / 1e6)
@@ -509,12 +510,13 @@ def run_spmv(args, rank, world, local_rank):
             "traffic": None if dia_bytes else traffic_for(args.workload),
             "kernel": ("nm::spmv_gather_kernel (warp per 32 rows, x gathered through L2)"
                        if kspmv.spmv_kernel(M) == "gather"
-                       else "nm::spmv_dia_kernel (diagonal form: fewer bytes than the CSR "
-                            "formula that `achieved` and `value` count)" if dia_bytes
+                       else "nm::spmv_dia_kernel (diagonal form)" if dia_bytes
                        else "nm::spmv_kernel (row-block CSR SpMV)"),
             "kernel_avg_us": round(kern_avg_ms * 1e3, 3),
+            # `achieved` counts these; `value` the bytes of the CSR formula, a
+            # rate of products, not of memory, where the kernel moves fewer
             "moved_bytes": moved,
-            "moved_frac": round(moved / (kern_avg_ms * 1e-3) / 1e9 / peak, 4),
+            "csr_formula_gbs": round(nbytes / (kern_avg_ms * 1e-3) / 1e9, 1),
         },
         "e2e": {
             "value": round(nbytes / (e2e_ms * 1e-3) / 1e9, 2), "unit": "GB/s",
@@ -644,7 +646,7 @@ def run_batch(args, rank, world, local_rank):
     line.update({
         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak,
                      "unit": "GB/s", "frac": round(achieved / peak, 4), "peak_source": peak_src,
-                     "traffic": None, "kernel": "nm::batch_spmv_kernel",
+                     "traffic": None, "kernel": "nm::batch_dia_kernel",
                      "kernel_avg_us": round(kern_avg_ms * 1e3, 3),
                      "reference_formula_gbs": round(
                          (12 * A.nnz + 8 * k * A.nrows + 8 * A.nrows) / (kern_avg_ms * 1e-3) / 1e9, 1)},
@@ -796,7 +798,9 @@ CG_PATHS = {0: "CUDA-graph chunks of 2 kernels per iteration (the p update forme
                "iteration)",
             4: "cluster solve (one 16-CTA thread-block cluster: the rows of A in shared "
                "memory, each CTA's halo of the direction kept current over distributed "
-               "shared memory, 2 hardware cluster barriers per iteration)"}
+               "shared memory, 2 hardware cluster barriers per iteration)",
+            5: "solve on the diagonal form (x, r and the direction on chip over all SMs, 2 "
+               "all-to-all exchanges of sums per iteration)"}
 
 
 def run_cg(args, rank, world, local_rank):
@@ -814,6 +818,7 @@ def run_cg(args, rank, world, local_rank):
     per_it = cg_iter_bytes(A.nnz, A.nrows, 8, 8)
     peak, peak_src = measured_peak()
     achieved = per_it * r["iters"] / (r["ms"] * 1e-3) / 1e9
+    on_chip = r["path_id"] in (3, 4, 5)
     ms_per = ms / args.steps
     config = {"workload": desc, "name": args.workload, "nrows": A.nrows, "nnz": A.nnz,
               "tol": 1e-8, "iters_per_solve": it_per_solve,
@@ -826,10 +831,15 @@ def run_cg(args, rank, world, local_rank):
     line = base_line(args, world, round(world * 1e3 / ms_per, 3), "solves/s", ms_per, precision,
                      config)
     line.update({
-        "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
-                     "frac": round(achieved / peak, 4), "peak_source": peak_src,
+        # the solves that keep matrix or vectors on chip (3, 4, 5) do not move
+        # the bytes of the formula: no share of the memory rate to give
+        "roofline": {"bound": "latency" if on_chip else "hbm",
+                     "achieved": None if on_chip else round(achieved, 1), "peak": peak,
+                     "unit": "GB/s", "frac": None if on_chip else round(achieved / peak, 4),
+                     "peak_source": peak_src,
                      "traffic": None, "kernel": "whole CG iteration (SpMV+p.Ap, x/r update, "
-                     "p update)", "bytes_per_iteration": per_it,
+                     "p update)", "formula_bytes_per_iteration": per_it,
+                     "formula_gbs": round(achieved, 1),
                      "us_per_iteration": round(r["ms"] * 1e3 / r["iters"], 3)},
         "e2e": {"value": round(1e3 / e2e_ms, 3), "unit": "solves/s",
                 "h2d_bytes_per_step": r["h2d"], "d2h_bytes_per_step": r["d2h"],
@@ -915,7 +925,11 @@ def run_engine(args, rank, world, local_rank):
     tb = 8 if precision == "fp64" else 4
     its = (c1["inner_iterations"] - c0["inner_iterations"]) / args.steps  # enqueued
     outer = st["outer"]
-    per_solve = st["iters"] * engine_iter_bytes(A.nnz, A.nrows, vb, tb) + \
+    # the one system has more than 131,072 rows on seven diagonals; the
+    # persistent step multiplies from its CSR arrays
+    dia = args.engine_mode != "persistent"
+    iter_bytes = engine_iter_bytes_dia if dia else engine_iter_bytes
+    per_solve = st["iters"] * iter_bytes(A.nnz, A.nrows, vb, tb) + \
         outer * engine_outer_bytes(A.nnz, A.nrows, tb)
     peak, peak_src = measured_peak()
     dev_s = (c1["s_device"] - c0["s_device"]) / args.steps
@@ -946,9 +960,10 @@ def run_engine(args, rank, world, local_rank):
                 "h2d_bytes_per_step": int(A.nnz * (12 + vb) + A.nrows * 16),
                 "d2h_bytes_per_step": int(A.nrows * 8), "ms_per_step": round(e_ms, 3),
                 "api": "BatchSolver.solve: admission from host arrays, steps, take"},
-        # per inner iteration of the one large system: SpMV, alpha, update, p
-        # update; one control kernel per 8-iteration body; the refinement steps
-        "gpu_launches": int((c1["inner_iterations"] - c0["inner_iterations"]) * 4 +
+        # per inner iteration of the one large system, in diagonal form: SpMV
+        # with alpha, update, p update; one control kernel per 8-iteration
+        # body; the refinement steps
+        "gpu_launches": int((c1["inner_iterations"] - c0["inner_iterations"]) * 3 +
                             (c1["inner_iterations"] - c0["inner_iterations"]) // 8 +
                             (c1["outer_launches"] - c0["outer_launches"]) * 6),
         "clocks": clk.summary(),
@@ -1119,7 +1134,7 @@ def run_serve(args, rank, world, local_rank):
                 "note": "the served loop is end to end by construction: every request's "
                         "matrix and b come from host memory and x goes back"},
         # at least SpMV, update, p update per inner iteration (alpha too while
-        # a large system is live), one control kernel per 8-iteration body,
+        # a large system without a diagonal form is live), one control kernel per 8-iteration body,
         # the refinement steps
         "gpu_launches": int((c1["inner_iterations"] - c0["inner_iterations"]) * 3 +
                             (c1["inner_iterations"] - c0["inner_iterations"]) // 8 +

@@ -68,8 +68,9 @@ typedef struct {
  * for it, if that copy takes at most 64 MB or a quarter of the free device
  * memory); else GATHER when at least 3/4 of the nonzeros lie in row blocks without x
  * windows and no row has more than 4096 nonzeros, else BLOCKS.  The
- * autotuner times all three.  CG and the batched engine always use the
- * row-block pipeline. */
+ * autotuner times them all.  CG and the batched engine have kernels of their
+ * own for matrices on at most 8 diagonals (see nm_cg_set_persistent and
+ * nm_solver_set_persistent) and use the row-block pipeline for the others. */
 enum nm_kernel { NM_KERNEL_AUTO = 1, NM_KERNEL_BLOCKS = 2, NM_KERNEL_GATHER = 3,
                  NM_KERNEL_SLICED = 4 };
 
@@ -172,6 +173,11 @@ int nm_csr_get_tuning(const nm_csr* A, nm_tuning* t);
 /* The plain-SpMV kernel nm_spmv runs on A under its tuning (AUTO resolved):
  * NM_KERNEL_BLOCKS, NM_KERNEL_GATHER or NM_KERNEL_SLICED. */
 int nm_csr_spmv_kernel(const nm_csr* A, int32_t* kernel);
+
+/* The diagonals nm_spmv runs A along (0: it runs from the CSR arrays), and the
+ * bytes of the matrix it reads then: masks and, where they vary along a
+ * diagonal, the values. */
+int nm_csr_diagonals(const nm_csr* A, int32_t* ndiag, int64_t* matrix_bytes);
 
 /* One timed candidate of nm_csr_autotune. */
 typedef struct {
@@ -335,7 +341,8 @@ typedef struct {
 
 /* Process-wide choice of how a step's inner iterations run: 0 (default) a
  * CUDA graph whose loop body launches the SpMV, update and p update of every
- * live system as kernels; 1 one persistent cooperative launch per step (the
+ * live system as kernels (systems of more than 131,072 rows on at most 8
+ * diagonals multiply along their diagonals); 1 one persistent cooperative launch per step (the
  * same phases separated by grid barriers, ending as soon as no system
  * iterates), when the device supports it.  Both give the same bits.  Other
  * values: NM_ERR_INVALID. */

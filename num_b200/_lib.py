@@ -64,6 +64,7 @@ _SIGNATURES = {
     "nm_csr_destroy": ([vp], C.c_int),
     "nm_csr_laplacian": ([i32, i32, C.c_int, C.POINTER(vp)], C.c_int),
     "nm_csr_spmv_kernel": ([vp, P_i32], C.c_int),
+    "nm_csr_diagonals": ([vp, P_i32, C.POINTER(C.c_int64)], C.c_int),
     "nm_csr_export": ([vp, vp, vp, vp], C.c_int),
     "nm_csr_info": ([vp, P_i32, P_i32, P_i32, P_i32, P_i32], C.c_int),
     "nm_csr_set_tuning": ([vp, C.POINTER(Tuning)], C.c_int),

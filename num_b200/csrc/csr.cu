@@ -548,6 +548,18 @@ extern "C" int nm_csr_spmv_kernel(const nm_csr* A, int32_t* kernel) {
     return NM_OK;
 }
 
+extern "C" int nm_csr_diagonals(const nm_csr* A, int32_t* ndiag, int64_t* matrix_bytes) {
+    nm::clear_error();
+    if (!A || !ndiag || !matrix_bytes)
+        return fail(NM_ERR_INVALID, "nm_csr_diagonals: NULL argument");
+    *ndiag = A->use_dia() ? A->dia.ndiag : 0;
+    *matrix_bytes = 0;
+    if (*ndiag > 0)
+        *matrix_bytes = (A->dia.ndiag <= 8 ? 1 : 2) * int64_t(A->nrows) +
+                        (A->dia.constant ? 0 : int64_t(nm::dtype_size(A->dtype)) * A->nnz);
+    return NM_OK;
+}
+
 extern "C" int nm_csr_get_tuning(const nm_csr* A, nm_tuning* t) {
     nm::clear_error();
     if (!A || !t) return fail(NM_ERR_INVALID, "nm_csr_get_tuning: NULL argument");
