@@ -185,7 +185,8 @@ int upload(nm_csr* A, const int32_t* rp, const int32_t* ci, const void* vals) {
     const size_t es = dtype_size(A->dtype);
     const int64_t nnz_pad = ((static_cast<int64_t>(A->nnz) + 7) & ~int64_t(7)) + 8;
     const size_t rp_len = size_t(A->nrows) + 1 + 8;
-    const int st = alloc_arrays(A, rp_len, size_t(nnz_pad), may_be_diagonal(rp, ci, A->nrows));
+    const int st = alloc_arrays(A, rp_len, size_t(nnz_pad),
+                                A->want_dia && may_be_diagonal(rp, ci, A->nrows));
     if (st != NM_OK) return st;
     const size_t rb = sizeof(int32_t) * rp_len, nzb = sizeof(int32_t) * size_t(A->nnz);
     unsigned char* base = reinterpret_cast<unsigned char*>(A->d_row_ptr);
@@ -348,17 +349,17 @@ nm_csr::~nm_csr() {
 
 using nm::fail;
 
-extern "C" int nm_csr_create(const int32_t* row_ptr, const int32_t* col_idx, const void* values,
-                             int dtype, int32_t nrows, int32_t ncols, nm_csr** out) {
-    nm::clear_error();
-    if (!out) return fail(NM_ERR_INVALID, "nm_csr_create: out is NULL");
+namespace nm {
+
+int create_csr(const int32_t* row_ptr, const int32_t* col_idx, const void* values, int dtype,
+               int32_t nrows, int32_t ncols, bool diagonal_form, nm_csr** out) {
     *out = nullptr;
     if (nrows <= 0 || ncols <= 0)
         return fail(NM_ERR_INVALID, "CrsMatrixHandle: non-positive dimensions");
-    if (nm::dtype_size(dtype) == 0) return fail(NM_ERR_TYPE, "nm_csr_create: unknown dtype %d", dtype);
+    if (dtype_size(dtype) == 0) return fail(NM_ERR_TYPE, "nm_csr_create: unknown dtype %d", dtype);
     if (!row_ptr || (row_ptr[nrows] > 0 && (!col_idx || !values)))
         return fail(NM_ERR_INVALID, "nm_csr_create: NULL array");
-    int st = nm::validate_csr(row_ptr, col_idx, nrows, ncols, "nm_csr_create");
+    int st = validate_csr(row_ptr, col_idx, nrows, ncols, "nm_csr_create");
     if (st != NM_OK) return st;
     auto* A = new nm_csr();
     cudaGetDevice(&A->device);
@@ -366,9 +367,19 @@ extern "C" int nm_csr_create(const int32_t* row_ptr, const int32_t* col_idx, con
     A->ncols = ncols;
     A->nnz = row_ptr[nrows];
     A->dtype = dtype;
+    A->want_dia = diagonal_form;
     A->tune = nm_tuning{0, 0, 0, 0, 0, 0};
-    nm::normalise_tuning(A->tune);
-    return nm::finish_create(A, row_ptr, col_idx, values, out);
+    normalise_tuning(A->tune);
+    return finish_create(A, row_ptr, col_idx, values, out);
+}
+
+}  // namespace nm
+
+extern "C" int nm_csr_create(const int32_t* row_ptr, const int32_t* col_idx, const void* values,
+                             int dtype, int32_t nrows, int32_t ncols, nm_csr** out) {
+    nm::clear_error();
+    if (!out) return fail(NM_ERR_INVALID, "nm_csr_create: out is NULL");
+    return nm::create_csr(row_ptr, col_idx, values, dtype, nrows, ncols, true, out);
 }
 
 extern "C" int nm_csr_create_batched(int32_t count, const int32_t* nrows, const int32_t* ncols,

@@ -161,6 +161,7 @@ struct nm_csr {
     // (found once, when the arrays are in place); d_dia_room lies behind the
     // values in their allocation (null where may_be_diagonal said no).
     nm::DiaForm dia;
+    bool want_dia = true;  // false: nothing would run from it
     unsigned char* d_dia_room = nullptr;
     // The plain SpMV runs on the diagonal form: it sums every row by one
     // thread, as the row-block kernel does for rows up to short_max.
@@ -208,6 +209,10 @@ constexpr int32_t kSellWindow = 65536;
 // Builds A's sliced copy for the gather kernel once (spmv.cu); NM_OK also
 // when the layout would pad too much (A->sell_ready stays false).
 int build_sell(nm_csr* A);
+// nm_csr_create; without `diagonal_form` for a matrix that only launch_spmv_rows
+// multiplies, which reads the CSR arrays.
+int create_csr(const int32_t* row_ptr, const int32_t* col_idx, const void* values, int dtype,
+               int32_t nrows, int32_t ncols, bool diagonal_form, nm_csr** out);
 // Whether a look at some rows leaves room for a diagonal form (dia.cu).
 bool may_be_diagonal(const int32_t* row_ptr, const int32_t* col_idx, int32_t nrows);
 // Looks for A's diagonal form (dia.cu) once its arrays are on the device: the

@@ -225,7 +225,8 @@ static int dist_build(const int32_t* rp, const int32_t* ci, const double* vals, 
                 }
                 srp.push_back(static_cast<int32_t>(sci.size()));
             }
-            return nm_csr_create(srp.data(), sci.data(), sv.data(), NM_F64, count, ncols_sub, outm);
+            return nm::create_csr(srp.data(), sci.data(), sv.data(), NM_F64, count, ncols_sub,
+                                  false, outm);
         };
         if (D->n_interior > 0) {
             int st = subset(0, D->n_interior, ln, &D->interior);

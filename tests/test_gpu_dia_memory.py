@@ -83,3 +83,23 @@ def test_engine_copies_values_only_out_of_plenty(kspmv, nearly_full):
         del S
     (x, i), (y, j) = out
     assert i["converged"] and i["iters"] == j["iters"] and np.array_equal(x, y)
+
+
+def test_row_subsets_hold_no_values_by_diagonal(kspmv):
+    """A rank's slice, and its interior and boundary rows as matrices of their
+    own: only the slice is multiplied along its diagonals."""
+    import ctypes as C
+
+    from num_b200 import _lib
+    A = _seven(N)
+    lib = _lib.load()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    before = torch.cuda.mem_get_info()[0]
+    h = C.c_void_p()
+    _lib.check(lib.nm_dist_create(A.row_ptr.ctypes.data, A.col_idx.ctypes.data,
+                                  A.values.ctypes.data, N, N, 0, 2, C.byref(h)))
+    used = before - torch.cuda.mem_get_info()[0]
+    lib.nm_dist_destroy(h)
+    csr, copy = 6 * A.nnz + 2 * N, 4 * 7 * N  # of half of the rows
+    assert 2 * csr + copy <= used < 2 * csr + 1.5 * copy
