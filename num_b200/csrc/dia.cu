@@ -233,6 +233,17 @@ int take_form(nm_csr* A) {
 // ---------------------------------------------------------------------------
 constexpr int kDiaThreads = 128;
 
+// A BF16 value, read only if `in`: as an `if` around the load of 16 bits it
+// becomes a branch, and a row's loads then wait for one another.
+__device__ __forceinline__ __nv_bfloat16 ld_bf16_cs_if(const __nv_bfloat16* p, bool in) {
+    unsigned short v;
+    asm("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.b16 %0, 0;\n\t"
+        "@q ld.global.cs.u16 %0, [%1];\n\t}"
+        : "=h"(v)
+        : "l"(p), "r"(unsigned(in)));
+    return __ushort_as_bfloat16(v);
+}
+
 template <typename V, typename X, typename A, int KC, bool CONST, int R>
 __global__ void __launch_bounds__(kDiaThreads)
     spmv_dia_kernel(const DiaView<A> D, int ndiag, const X* __restrict__ x, X* __restrict__ y) {
@@ -276,10 +287,12 @@ __global__ void __launch_bounds__(kDiaThreads)
                 for (int k = 0; k < KC; ++k) {
                     xs[r][k] = A(0);
                     vs[r][k] = cv[k];
-                    if (m[r] >> k & 1u) {
-                        xs[r][k] = static_cast<A>(__ldg(xp[k] + r * kDiaThreads));
-                        if constexpr (!CONST) vs[r][k] = widen<V, A>(ld_value_cs(vp + k * D.ld));
-                    }
+                    const bool in = m[r] >> k & 1u;
+                    if (in) xs[r][k] = static_cast<A>(__ldg(xp[k] + r * kDiaThreads));
+                    if constexpr (!CONST && sizeof(V) == 2)
+                        vs[r][k] = __bfloat162float(ld_bf16_cs_if(vp + k * D.ld, in));
+                    else if constexpr (!CONST)
+                        if (in) vs[r][k] = widen<V, A>(ld_value_cs(vp + k * D.ld));
                 }
             }
         }
@@ -343,6 +356,7 @@ int launch_dia_t(const nm_csr* M, const void* x, void* y, cudaStream_t s) {
     if (nd <= 7) return launch_dia_k<V, X, A, 7>(M, xx, yy, s);
     if (nd <= 8) return launch_dia_k<V, X, A, 8>(M, xx, yy, s);
     if (nd <= 9) return launch_dia_k<V, X, A, 9>(M, xx, yy, s);  // 16-bit masks from here on
+    if (nd <= 12) return launch_dia_k<V, X, A, 12>(M, xx, yy, s);
     return launch_dia_k<V, X, A, kDiaMax>(M, xx, yy, s);
 }
 
