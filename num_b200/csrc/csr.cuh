@@ -222,8 +222,9 @@ int search_dia_form(const nm_csr* A);
 int take_dia_form(nm_csr* A);
 // y = A x on the diagonal form.
 int launch_spmv_dia(const nm_csr* A, const void* x, void* y, cudaStream_t stream);
-// Y = A X (row-major, k columns; vec2: k even and X, Y 16-byte aligned) on the
-// diagonal form.
+// Whether Y = A X (row-major, k columns; vec2: k even and X, Y 16-byte aligned)
+// runs from the diagonal form; and that product.
+bool batch_on_diagonals(const nm_csr* A, int32_t k, bool vec2);
 int launch_batch_dia(const nm_csr* A, const double* X, double* Y, int32_t k, bool vec2,
                      cudaStream_t stream);
 // Drops A's cached CG workspace (its graphs hold the current descriptors).

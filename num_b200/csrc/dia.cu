@@ -452,9 +452,12 @@ __global__ void __launch_bounds__(kDiaBatchThreads)
     }
 }
 
-// The same for more than 8 diagonals: rows of a matrix with that many use few
-// of them (a periodic grid's wrap-around diagonals), so a row's diagonals are
-// taken from its mask, kDiaBits at a time, instead of asking each in turn.
+// The same for more than 8 diagonals of which a row uses few (a periodic grid's
+// wrap-around diagonals): a row's diagonals are taken from its mask, kDiaBits
+// at a time, instead of asking each in turn.  Where rows have nearly all of
+// them (mostly_full) the unrolled kernel takes those matrices too: 16
+// varying diagonals, 300,000 rows, k = 9 1.4 times as fast, k = 63 1.7 times;
+// with 0.6 of them there it is 0.9 times as fast.
 constexpr int kDiaBits = 6;
 
 template <bool CONST, int VEC>
@@ -515,12 +518,17 @@ __global__ void __launch_bounds__(kDiaBatchThreads)
     }
 }
 
+// Nearly every row has an entry on every diagonal (7 in 8).
+bool mostly_full(const nm_csr* A) {
+    return 8 * int64_t(A->nnz) >= 7 * int64_t(A->dia.ndiag) * A->nrows;
+}
+
 template <int KC, bool CONST, int VEC>
 void launch_batch_dia_t(const nm_csr* A, const DiaBatchShape& b, const double* X, double* Y,
                         int32_t k, cudaStream_t s) {
     const auto D = dia_view<double>(A->dia, A->nrows);
     const unsigned g = static_cast<unsigned>(b.grid);
-    if constexpr (KC > 8)
+    if (KC > 8 && !mostly_full(A))
         batch_dia_bits_kernel<CONST, VEC><<<g, kDiaBatchThreads, 0, s>>>(
             D, k, b.lg, b.chunk_cols, b.nchunk, b.run, X, Y);
     else
@@ -595,6 +603,14 @@ int launch_spmv_dia(const nm_csr* A, const void* x, void* y, cudaStream_t s) {
     }
 }
 
+bool batch_on_diagonals(const nm_csr* A, int32_t k, bool vec2) {
+    if (A->dia.ndiag == 0) return false;
+    const int vec = vec2 ? 2 : 1;
+    if (csr_batch_shape(k, vec).ch < 2) return true;
+    return dia_batch_takes(A->nrows, A->dia.ndiag, mostly_full(A), A->dia.constant, k, vec,
+                           dia_batch_shape(A->nrows, k, vec, sm_count()));
+}
+
 int launch_batch_dia(const nm_csr* A, const double* X, double* Y, int32_t k, bool vec2,
                      cudaStream_t s) {
     const int nd = A->dia.ndiag;
@@ -604,6 +620,8 @@ int launch_batch_dia(const nm_csr* A, const double* X, double* Y, int32_t k, boo
     else if (nd <= 5) launch_batch_dia_k<5>(A, b, X, Y, k, vec2, s);
     else if (nd <= 7) launch_batch_dia_k<7>(A, b, X, Y, k, vec2, s);
     else if (nd <= 8) launch_batch_dia_k<8>(A, b, X, Y, k, vec2, s);
+    else if (nd <= 9) launch_batch_dia_k<9>(A, b, X, Y, k, vec2, s);
+    else if (nd <= 12) launch_batch_dia_k<12>(A, b, X, Y, k, vec2, s);
     else launch_batch_dia_k<kDiaMax>(A, b, X, Y, k, vec2, s);
     NM_CHECK_LAUNCH();
     return NM_OK;

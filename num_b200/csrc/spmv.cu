@@ -1,4 +1,5 @@
 // spmv.cu -- plain SpMV and multi-RHS SpMV kernels and their launchers.
+#include "batch_shape.cuh"
 #include "spmv.cuh"
 
 #include <algorithm>
@@ -476,7 +477,6 @@ int launch_spmv(const nm_csr* A, const void* x, void* y, cudaStream_t s) {
 // matrix entries of a row are read once per column pass and broadcast to the
 // group; X rows are read as contiguous segments (coalesced).
 // ---------------------------------------------------------------------------
-constexpr int kBatchChunks = 4;  // most column chunks per lane in one pass
 constexpr int kBatchNz = 4;      // nonzeros whose X rows are loaded together
 
 template <int VEC, int CH>
@@ -721,7 +721,7 @@ template <int VEC>
 static void launch_batch_v(const nm_csr* A, const double* X, double* Y, int32_t k, int tpr_log2,
                            int ch, int grid, cudaStream_t s) {
     if (ch >= 4) launch_batch_t<VEC, 4>(A, X, Y, k, tpr_log2, grid, s);
-    else if (ch == 2 || ch == 3) launch_batch_t<VEC, 2>(A, X, Y, k, tpr_log2, grid, s);
+    else if (ch == 2) launch_batch_t<VEC, 2>(A, X, Y, k, tpr_log2, grid, s);
     else launch_batch_t<VEC, 1>(A, X, Y, k, tpr_log2, grid, s);
 }
 
@@ -730,13 +730,9 @@ static int launch_batch(const nm_csr* A, const double* X, double* Y, int32_t k, 
                       (reinterpret_cast<uintptr_t>(Y) % 16 == 0);
     // Matrices in diagonal form have kernels of their own (dia.cu); like those
     // below they sum every (row, column) serially in CSR order.
-    if (A->dia.ndiag > 0) return launch_batch_dia(A, X, Y, k, vec2, s);
-    const int vec = vec2 ? 2 : 1;
-    const int groups = (k + vec - 1) / vec;  // lane-columns needed for one pass
-    int tpr_log2 = 0;
-    while ((1 << tpr_log2) < groups && tpr_log2 < 5) ++tpr_log2;
-    // column chunks per lane: enough for k in one pass, at most kBatchChunks
-    const int ch = std::min(kBatchChunks, (groups + (1 << tpr_log2) - 1) >> tpr_log2);
+    if (batch_on_diagonals(A, k, vec2)) return launch_batch_dia(A, X, Y, k, vec2, s);
+    const CsrBatchShape c = csr_batch_shape(k, vec2 ? 2 : 1);
+    const int tpr_log2 = c.tpr_log2, ch = c.ch;
     const int64_t threads = int64_t(A->nrows) << tpr_log2;
     const int64_t grid = (threads + kThreads - 1) / kThreads;
     if (grid > INT32_MAX) return fail(NM_ERR_INVALID, "batch_spmv: problem too large");
