@@ -274,7 +274,7 @@ int nm_scale(int64_t n, double alpha, double* x, void* stream);
  * give the same iterates, bit for bit (every dot product is summed in one
  * fixed order: per row block or 256-row tile, then over the blocks), but that
  * above 262,144 rows the solve on the diagonal form and the graph each have
- * their own.  Other
+ * their own (that of the first also depends on the number of SMs).  Other
  * values: NM_ERR_INVALID.  No reference counterpart (an implementation
  * switch). */
 int nm_cg_set_persistent(int32_t enable);

@@ -36,7 +36,8 @@
 //    division in all 512 threads costs 300 cycles of the FP64 pipe.
 //  * Up to kDiaCgTileSums tiles the sums are per tile, in the order every
 //    other CG path uses (reduce256 over the tiles), so the bits are theirs;
-//    beyond, per CTA (its tile sums by a warp's shuffle tree).
+//    beyond, per CTA (its tile sums by a warp's shuffle tree), so that they
+//    also depend on the number of SMs.
 //
 // Every wait is bounded (kWaitLimitNs); a CTA that gives up sets the error
 // word and the state to kCgDeviceError and leaves, and the others give up in
