@@ -158,19 +158,20 @@ int validate_csr(const int32_t* rp, const int32_t* ci, int32_t nrows, int32_t nc
 }
 
 // The matrix's arrays (rp_len row offsets, nnz_pad columns and values) and,
-// where it may have a diagonal form, room for the search for it and for its
-// masks: one allocation.
-int alloc_arrays(nm_csr* A, size_t rp_len, size_t nnz_pad, bool dia_room) {
+// where it may have a diagonal form, room for the search for it, for its
+// masks and for `copy` bytes of values by diagonal: one allocation.
+int alloc_arrays(nm_csr* A, size_t rp_len, size_t nnz_pad, bool dia_room, size_t copy) {
     auto up = [](size_t b) { return (b + 255) & ~size_t(255); };
     const size_t rb = up(sizeof(int32_t) * rp_len), cb = up(sizeof(int32_t) * nnz_pad);
     const size_t vb = up(dtype_size(A->dtype) * nnz_pad);
-    const size_t db = dia_room ? kDiaTableBytes + 2 * size_t(A->nrows) : 0;
+    const size_t db = dia_room ? kDiaTableBytes + dia_mask_room(A->nrows) + copy : 0;
     unsigned char* base = nullptr;
     NM_CUDA_TRY(cudaMalloc(&base, rb + cb + vb + db));
     A->d_row_ptr = reinterpret_cast<int32_t*>(base);
     A->d_col_idx = reinterpret_cast<int32_t*>(base + rb);
     A->d_values = base + rb + cb;
     A->d_dia_room = dia_room ? base + rb + cb + vb : nullptr;
+    A->dia_copy_room = dia_room ? copy : 0;
     return NM_OK;
 }
 
@@ -185,8 +186,10 @@ int upload(nm_csr* A, const int32_t* rp, const int32_t* ci, const void* vals) {
     const size_t es = dtype_size(A->dtype);
     const int64_t nnz_pad = ((static_cast<int64_t>(A->nnz) + 7) & ~int64_t(7)) + 8;
     const size_t rp_len = size_t(A->nrows) + 1 + 8;
-    const int st = alloc_arrays(A, rp_len, size_t(nnz_pad),
-                                A->want_dia && may_be_diagonal(rp, ci, A->nrows));
+    size_t copy = 0;
+    const bool dia = A->want_dia && may_be_diagonal(rp, ci, vals, es, A->nrows, &copy);
+    if (copy > kCopyAlways) copy = 0;  // an allocation of its own, if at all
+    const int st = alloc_arrays(A, rp_len, size_t(nnz_pad), dia, copy);
     if (st != NM_OK) return st;
     const size_t rb = sizeof(int32_t) * rp_len, nzb = sizeof(int32_t) * size_t(A->nnz);
     unsigned char* base = reinterpret_cast<unsigned char*>(A->d_row_ptr);
@@ -344,7 +347,7 @@ nm_csr::~nm_csr() {
     if (d_sell_len) cudaFree(d_sell_len);
     if (d_sell_col) cudaFree(d_sell_col);
     if (d_sell_val) cudaFree(d_sell_val);
-    if (dia.d_val) cudaFree(dia.d_val);
+    if (dia.own_val) cudaFree(dia.d_val);
 }
 
 using nm::fail;
@@ -470,10 +473,13 @@ extern "C" int nm_csr_laplacian(int32_t dim, int32_t L, int dtype, nm_csr** out)
         // Same allocation and padding as an uploaded matrix.
         const int64_t nnz_pad = ((nnz + 7) & ~int64_t(7)) + 8;
         const int64_t rp_len = n + 1 + 8;
-        int st = nm::alloc_arrays(A, size_t(rp_len), size_t(nnz_pad), true);
+        int st = nm::alloc_arrays(A, size_t(rp_len), size_t(nnz_pad), true, 0);
         if (st != NM_OK) return st;
+        // The diagonal form is known (a grid of one point has fewer diagonals
+        // than directions: that one is searched).
+        unsigned char* mask = L > 1 ? A->d_dia_room + nm::kDiaTableBytes : nullptr;
         st = nm::launch_laplacian(dim, L, dtype, A->d_row_ptr, rp_len, A->d_col_idx,
-                                  A->d_values, nnz_pad, nullptr);
+                                  A->d_values, nnz_pad, mask, nullptr);
         if (st != NM_OK) return st;
         // The row-block partition is built on the host from row_ptr and the
         // columns (as for an uploaded matrix): read them back once.
@@ -483,9 +489,11 @@ extern "C" int nm_csr_laplacian(int32_t dim, int32_t L, int dtype, nm_csr** out)
                                cudaMemcpyDeviceToHost));
         NM_CUDA_TRY(cudaMemcpy(A->h_col_idx.data(), A->d_col_idx, sizeof(int32_t) * size_t(nnz),
                                cudaMemcpyDeviceToHost));
-        st = nm::search_dia_form(A);
+        if (!mask) st = nm::search_dia_form(A);
         if (st == NM_OK) st = nm::rebuild_blocks(A);
-        return st == NM_OK ? nm::take_dia_form(A) : st;
+        if (st != NM_OK || !mask) return st != NM_OK ? st : nm::take_dia_form(A);
+        A->dia = nm::laplacian_form(dim, L, mask);
+        return NM_OK;
     };
     const int st = build();
     if (st != NM_OK) {

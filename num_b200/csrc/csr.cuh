@@ -1,8 +1,8 @@
 // csr.cuh -- internal layout of a device CSR matrix.
 //
 // HBM layout (256-byte aligned), two allocations: the first three with the room
-// of DiaForm behind them, and the last two (32^3 varying coefficients, upload:
-// 1.74 ms, 2.06 with the first three apart):
+// of DiaForm behind them, and the last two (30^3 varying coefficients, upload:
+// 1.48 ms; 1.90 with an allocation each and for the values by diagonal):
 //   row_ptr  int32[nrows + 1 + 8]  pad = nnz
 //   col_idx  int32[nnz_pad]        nnz_pad = round_up(nnz, 8) + 8, pad = column 0
 //   values   V[nnz_pad]            pad = 0
@@ -73,11 +73,15 @@ struct DiaForm {
     double cval[kDiaMax] = {};
     void* d_mask = nullptr;  // uint8_t[nrows] up to 8 diagonals, else uint16_t[nrows]
     void* d_val = nullptr;   // values [ndiag][ld], the matrix's type
+    bool own_val = false;    // d_val is an allocation of its own
 };
 
 // Room behind the values for the search for that form (dia.cu); the masks
-// follow it there.
+// follow it there, and values by diagonal of up to kCopyAlways bytes where a
+// look at some rows says that they vary.
 constexpr size_t kDiaTableBytes = 512;
+inline size_t dia_mask_room(int32_t nrows) { return (2 * size_t(nrows) + 255) & ~size_t(255); }
+inline int64_t dia_ld(int32_t nrows) { return (int64_t(nrows) + 31) & ~int64_t(31); }
 
 // Default row-block parameters.
 constexpr int kDefaultTile = 2048;
@@ -163,6 +167,7 @@ struct nm_csr {
     nm::DiaForm dia;
     bool want_dia = true;  // false: nothing would run from it
     unsigned char* d_dia_room = nullptr;
+    size_t dia_copy_room = 0;  // bytes for values by diagonal there
     // The plain SpMV runs on the diagonal form: it sums every row by one
     // thread, as the row-block kernel does for rows up to short_max.
     bool use_dia() const {
@@ -213,8 +218,11 @@ int build_sell(nm_csr* A);
 // multiplies, which reads the CSR arrays.
 int create_csr(const int32_t* row_ptr, const int32_t* col_idx, const void* values, int dtype,
                int32_t nrows, int32_t ncols, bool diagonal_form, nm_csr** out);
-// Whether a look at some rows leaves room for a diagonal form (dia.cu).
-bool may_be_diagonal(const int32_t* row_ptr, const int32_t* col_idx, int32_t nrows);
+// Whether a look at some rows leaves a diagonal form possible (dia.cu);
+// *copy_bytes: what its values by diagonal would take, 0 where the look sees
+// them constant.
+bool may_be_diagonal(const int32_t* row_ptr, const int32_t* col_idx, const void* values,
+                     size_t value_bytes, int32_t nrows, size_t* copy_bytes);
 // Looks for A's diagonal form (dia.cu) once its arrays are on the device: the
 // search is started, and its result taken after the host's work on the row
 // blocks, under which it runs.  NM_OK also when A has none.
@@ -233,7 +241,9 @@ void reset_cg(nm_csr* A);
 int64_t stencil_nnz(int dim, int32_t L);
 // Writes that Laplacian's row_ptr (rp_len entries, those past the last row =
 // nnz), col_idx and values (dtype; nnz_pad entries each, those past nnz = 0)
-// into device arrays on `stream` (gen.cu).
+// into device arrays on `stream` (gen.cu), and, where mask is set, the masks of
+// its diagonal form, whose diagonals ascend: laplacian_form.
 int launch_laplacian(int dim, int32_t L, int dtype, int32_t* rp, int64_t rp_len, int32_t* ci,
-                     void* val, int64_t nnz_pad, cudaStream_t stream);
+                     void* val, int64_t nnz_pad, uint8_t* mask, cudaStream_t stream);
+DiaForm laplacian_form(int dim, int32_t L, unsigned char* mask);
 }  // namespace nm

@@ -178,7 +178,7 @@ int take_form(nm_csr* A) {
     if (!constant && 2 * int64_t(A->nnz) < int64_t(nd) * n) return NM_OK;  // mostly padding
     DiaForm f;
     f.constant = constant;
-    f.ld = (int64_t(n) + 31) & ~int64_t(31);
+    f.ld = dia_ld(n);
     DiaOffsets o{};
     for (int k = 0; k < kDiaMax; ++k) {
         f.off[k] = o.off[k] = k < nd ? h.off[order[k]] : 0;
@@ -194,8 +194,14 @@ int take_form(nm_csr* A) {
         }
     }
     f.d_mask = A->d_dia_room + kDiaTableBytes;
-    if (!constant && !alloc_copy(&f.d_val, sizeof(V) * size_t(nd) * size_t(f.ld)))
-        return NM_OK;  // no room beside the CSR arrays: they serve alone
+    if (!constant) {
+        const size_t need = sizeof(V) * size_t(nd) * size_t(f.ld);
+        f.own_val = need > A->dia_copy_room;
+        if (!f.own_val)
+            f.d_val = A->d_dia_room + kDiaTableBytes + dia_mask_room(n);
+        else if (!alloc_copy(&f.d_val, need))
+            return NM_OK;  // no room beside the CSR arrays: they serve alone
+    }
     if (nd <= 8)
         dia_fill_kernel<V, uint8_t><<<static_cast<int>(want), kThreads>>>(
             A->d_row_ptr, A->d_col_idx, vals, n, o, static_cast<uint8_t*>(f.d_mask),
@@ -215,7 +221,7 @@ int take_form(nm_csr* A) {
         ragged = 32 * h.pairs > (unsigned long long)A->nnz * 5 / 4 + 32 * kDiaMax;
     }
     if (e != cudaSuccess || ragged) {
-        if (f.d_val) cudaFree(f.d_val);
+        if (f.own_val) cudaFree(f.d_val);
         NM_CUDA_TRY(e);
         return NM_OK;
     }
@@ -549,8 +555,11 @@ void launch_batch_dia_k(const nm_csr* A, const DiaBatchShape& b, const double* X
 }
 
 // The diagonals of some rows, on the host: a matrix of scattered columns shows
-// more than kDiaMax there (false) and costs nothing more.
-bool look_at_rows(const int32_t* rp, const int32_t* ci, int32_t nrows, DiaSeed* seed) {
+// more than kDiaMax there (false) and costs nothing more.  *varying: the looked
+// at entries of a diagonal differ (where the values, of es bytes, are given).
+bool look_at_rows(const int32_t* rp, const int32_t* ci, int32_t nrows, DiaSeed* seed,
+                  const void* vals = nullptr, size_t es = 0, bool* varying = nullptr) {
+    const char* v = static_cast<const char*>(vals);
     if (nrows == 0 || rp[nrows] == 0) return false;
     constexpr int kLook = 64;
     for (int q = 0; q < kLook; ++q) {
@@ -558,8 +567,11 @@ bool look_at_rows(const int32_t* rp, const int32_t* ci, int32_t nrows, DiaSeed* 
         if (rp[r + 1] - rp[r] > kDiaMax) return false;
         for (int32_t z = rp[r]; z < rp[r + 1]; ++z) {
             const int32_t d = ci[z] - r;
-            if (std::find(seed->off, seed->off + seed->count, d) != seed->off + seed->count)
+            const int s = int(std::find(seed->off, seed->off + seed->count, d) - seed->off);
+            if (s < seed->count) {
+                if (v) *varying |= std::memcmp(v + es * z, v + es * seed->at[s], es) != 0;
                 continue;
+            }
             if (seed->count == kDiaMax) return false;
             seed->off[seed->count] = d;
             seed->at[seed->count++] = z;
@@ -570,9 +582,17 @@ bool look_at_rows(const int32_t* rp, const int32_t* ci, int32_t nrows, DiaSeed* 
 
 }  // namespace
 
-bool may_be_diagonal(const int32_t* row_ptr, const int32_t* col_idx, int32_t nrows) {
+bool may_be_diagonal(const int32_t* row_ptr, const int32_t* col_idx, const void* values,
+                     size_t value_bytes, int32_t nrows, size_t* copy_bytes) {
     DiaSeed seed{};
-    return look_at_rows(row_ptr, col_idx, nrows, &seed);
+    bool varying = false;
+    const bool may =
+        look_at_rows(row_ptr, col_idx, nrows, &seed, values, value_bytes, &varying);
+    const int64_t nnz = nrows > 0 ? row_ptr[nrows] : 0;
+    *copy_bytes = may && varying && 2 * nnz >= int64_t(seed.count) * nrows
+                      ? value_bytes * size_t(seed.count) * size_t(dia_ld(nrows))
+                      : 0;
+    return may;
 }
 
 int search_dia_form(const nm_csr* A) {

@@ -49,14 +49,16 @@ namespace {
 // group; the CTA then writes the group's contiguous column / value range with
 // consecutive threads on consecutive elements (full-sector stores), and CTA 0
 // fills the row_ptr padding past row n - 1 with nnz and the columns and values
-// past nnz with zeros.
+// past nnz with zeros.  mask (may be null): the row's diagonals, bit k for the
+// k-th of -L^2 (3-D), -L, -1, 0, 1, L, L^2 (3-D).
 constexpr int kGenRows = 256;
 constexpr int kGenMaxNz = 7;  // nonzeros of a 7-point row
 
 template <typename V>
 __global__ void __launch_bounds__(kGenRows)
     laplacian_kernel(int dim, uint32_t L, uint32_t n, int64_t rp_len, int32_t* __restrict__ rp,
-                     int32_t* __restrict__ ci, V* __restrict__ val, int64_t nnz_pad, V diag, V off) {
+                     int32_t* __restrict__ ci, V* __restrict__ val, int64_t nnz_pad,
+                     uint8_t* __restrict__ mask, V diag, V off) {
     __shared__ int32_t s_ci[kGenRows * kGenMaxNz];
     __shared__ V s_v[kGenRows * kGenMaxNz];
     const uint32_t LL = L * L;
@@ -80,6 +82,11 @@ __global__ void __launch_bounds__(kGenRows)
             if (x + 1 < L) { s_ci[k] = int32_t(i + 1); s_v[k] = off; ++k; }
             if (y + 1 < L) { s_ci[k] = int32_t(i + L); s_v[k] = off; ++k; }
             if (dim == 3 && z + 1 < L) { s_ci[k] = int32_t(i + LL); s_v[k] = off; }
+            if (mask) {
+                uint32_t m = (y > 0) | (x > 0) << 1 | 1u << 2 | (x + 1 < L) << 3 | (y + 1 < L) << 4;
+                if (dim == 3) m = (z > 0) | m << 1 | (z + 1 < L) << 6;
+                mask[i] = static_cast<uint8_t>(m);
+            }
         }
         __syncthreads();
         const int cnt = static_cast<int>(stencil_before(dim, L, n, r1) - base);
@@ -102,7 +109,7 @@ __global__ void __launch_bounds__(kGenRows)
 
 template <typename V>
 int launch_t(int dim, int32_t L, int32_t n, int64_t rp_len, int32_t* rp, int32_t* ci, void* val,
-             int64_t nnz_pad, V diag, V off, cudaStream_t s) {
+             int64_t nnz_pad, uint8_t* mask, V diag, V off, cudaStream_t s) {
     if (rp_len < int64_t(n) + 1 || rp_len - n > kGenRows)
         return fail(NM_ERR_INVALID, "laplacian: row_ptr length %lld for %d rows", (long long)rp_len, n);
     if (nnz_pad - stencil_nnz(dim, L) > kGenRows)
@@ -110,23 +117,38 @@ int launch_t(int dim, int32_t L, int32_t n, int64_t rp_len, int32_t* rp, int32_t
     const int64_t blocks =
         std::min<int64_t>((int64_t(n) + kGenRows - 1) / kGenRows, int64_t(sm_count()) * 8);
     laplacian_kernel<V><<<static_cast<int>(blocks), kGenRows, 0, s>>>(
-        dim, uint32_t(L), uint32_t(n), rp_len, rp, ci, static_cast<V*>(val), nnz_pad, diag, off);
+        dim, uint32_t(L), uint32_t(n), rp_len, rp, ci, static_cast<V*>(val), nnz_pad, mask, diag, off);
     NM_CHECK_LAUNCH();
     return NM_OK;
 }
 
 }  // namespace
 
+DiaForm laplacian_form(int dim, int32_t L, unsigned char* mask) {
+    DiaForm f;
+    const int32_t n = dim == 2 ? L * L : L * L * L, LL = dim == 2 ? 0 : L * L;
+    const int32_t off[7] = {-LL, -L, -1, 0, 1, L, LL};
+    f.ndiag = 2 * dim + 1;
+    for (int k = 0; k < f.ndiag; ++k) {
+        f.off[k] = off[k + (dim == 2)];
+        f.cval[k] = f.off[k] == 0 ? 2.0 * dim : -1.0;
+    }
+    f.constant = true;
+    f.ld = dia_ld(n);
+    f.d_mask = mask;
+    return f;
+}
+
 int launch_laplacian(int dim, int32_t L, int dtype, int32_t* rp, int64_t rp_len, int32_t* ci,
-                     void* val, int64_t nnz_pad, cudaStream_t s) {
+                     void* val, int64_t nnz_pad, uint8_t* mask, cudaStream_t s) {
     const int32_t n = dim == 2 ? L * L : L * L * L;
     const double d = dim == 2 ? 4.0 : 6.0;
     switch (dtype) {
-        case NM_F64: return launch_t<double>(dim, L, n, rp_len, rp, ci, val, nnz_pad, d, -1.0, s);
+        case NM_F64: return launch_t<double>(dim, L, n, rp_len, rp, ci, val, nnz_pad, mask, d, -1.0, s);
         case NM_F32:
-            return launch_t<float>(dim, L, n, rp_len, rp, ci, val, nnz_pad, float(d), -1.0f, s);
+            return launch_t<float>(dim, L, n, rp_len, rp, ci, val, nnz_pad, mask, float(d), -1.0f, s);
         case NM_BF16:
-            return launch_t<__nv_bfloat16>(dim, L, n, rp_len, rp, ci, val, nnz_pad,
+            return launch_t<__nv_bfloat16>(dim, L, n, rp_len, rp, ci, val, nnz_pad, mask,
                                            __float2bfloat16_rn(float(d)),
                                            __float2bfloat16_rn(-1.0f), s);
         default: return fail(NM_ERR_TYPE, "laplacian: unknown dtype %d", dtype);

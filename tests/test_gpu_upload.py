@@ -59,3 +59,28 @@ def test_upload_without_nonzeros(kspmv):
     y = torch.full((300,), float("nan"), dtype=torch.float64, device="cuda")
     kspmv.spmv(M, torch.ones(5, dtype=torch.float64, device="cuda"), y)
     assert torch.count_nonzero(y).item() == 0
+
+
+@pytest.mark.parametrize("dim,L", [(2, 1), (2, 2), (2, 3), (2, 17), (3, 1), (3, 2), (3, 3), (3, 9)])
+@pytest.mark.parametrize("precision", ["fp64", "fp32", "bf16"])
+def test_assembled_laplacian_has_the_uploaded_ones_form(kspmv, oracle, dim, L, precision):
+    import ctypes as C
+
+    from num_b200 import _lib
+    A = gen.laplacian_2d(L) if dim == 2 else gen.laplacian_3d(L)
+    handles = [kspmv.laplacian(dim, L, precision=precision),
+               kspmv.upload_csr(A.row_ptr, A.col_idx, A.values, A.nrows, A.ncols,
+                                precision=precision)]
+    x = ((np.arange(A.ncols) % 17) - 8) / 8.0
+    want = oracle.spmv(A.row_ptr, A.col_idx, A.values, x)
+    seen = []
+    for M in handles:
+        nd, b = C.c_int32(), C.c_int64()
+        _lib.check(_lib.load().nm_csr_diagonals(M._h, C.byref(nd), C.byref(b)))
+        seen.append((nd.value, b.value))
+        xt = torch.tensor(x, dtype=torch.float64 if precision == "fp64" else torch.float32,
+                          device="cuda")
+        y = torch.full_like(xt, float("nan"))
+        kspmv.spmv(M, xt, y)
+        assert np.array_equal(y.cpu().numpy().astype(np.float64), want)
+    assert seen[0] == seen[1] and seen[0][0] == (2 * dim + 1 if L > 1 else 1)
