@@ -159,19 +159,27 @@ int validate_csr(const int32_t* rp, const int32_t* ci, int32_t nrows, int32_t nc
 
 // The matrix's arrays (rp_len row offsets, nnz_pad columns and values) and,
 // where it may have a diagonal form, room for the search for it, for its
-// masks and for `copy` bytes of values by diagonal: one allocation.
+// masks and for `copy` bytes of values by diagonal: one allocation, without
+// the last where the device has no room for them.  (They stay unused where the
+// search finds that the matrix has no such form after all.)
 int alloc_arrays(nm_csr* A, size_t rp_len, size_t nnz_pad, bool dia_room, size_t copy) {
     auto up = [](size_t b) { return (b + 255) & ~size_t(255); };
     const size_t rb = up(sizeof(int32_t) * rp_len), cb = up(sizeof(int32_t) * nnz_pad);
     const size_t vb = up(dtype_size(A->dtype) * nnz_pad);
-    const size_t db = dia_room ? kDiaTableBytes + dia_mask_room(A->nrows) + copy : 0;
+    const size_t db = dia_room ? kDiaTableBytes + dia_mask_room(A->nrows) : 0;
     unsigned char* base = nullptr;
-    NM_CUDA_TRY(cudaMalloc(&base, rb + cb + vb + db));
+    if (!dia_room) copy = 0;
+    if (copy > 0 && cudaMalloc(&base, rb + cb + vb + db + copy) != cudaSuccess) {
+        cudaGetLastError();
+        base = nullptr;
+        copy = 0;
+    }
+    if (!base) NM_CUDA_TRY(cudaMalloc(&base, rb + cb + vb + db));
     A->d_row_ptr = reinterpret_cast<int32_t*>(base);
     A->d_col_idx = reinterpret_cast<int32_t*>(base + rb);
     A->d_values = base + rb + cb;
     A->d_dia_room = dia_room ? base + rb + cb + vb : nullptr;
-    A->dia_copy_room = dia_room ? copy : 0;
+    A->dia_copy_room = copy;
     return NM_OK;
 }
 

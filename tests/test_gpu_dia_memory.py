@@ -63,6 +63,20 @@ def test_upload_copies_values_only_out_of_plenty(kspmv, oracle, nearly_full):
     assert used[1] < csr + copy   # ... and without: it would take half of what is left
 
 
+def test_upload_where_only_the_csr_arrays_fit(kspmv, oracle, nearly_full):
+    # 56 MB of values by diagonal, below what is asked about first
+    n = 1_000_000
+    A = _seven(n)
+    x = torch.from_numpy(np.random.default_rng(4).uniform(-1, 1, n)).cuda()
+    y = torch.full_like(x, float("nan"))
+    csr, copy = 12 * A.nnz + 4 * n, 8 * 7 * n
+    nearly_full(csr + copy // 2)
+    M = kspmv.upload_csr(A.row_ptr, A.col_idx, A.values, n, n)
+    kspmv.spmv(M, x, y)
+    assert np.array_equal(y.cpu().numpy(),
+                          oracle.spmv(A.row_ptr, A.col_idx, A.values, x.cpu().numpy()))
+
+
 def test_engine_copies_values_only_out_of_plenty(kspmv, nearly_full):
     from num_b200.solver import BatchSolver
     A = _seven(2 * N)
